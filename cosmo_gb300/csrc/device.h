@@ -186,6 +186,7 @@ struct SpmmCandidate {
 
 struct VirtualOp;
 struct TiledOp;
+struct FactoredOp;
 struct Hamiltonian {
   int device = 0;
   int precision = CG_PREC_FP64;
@@ -200,6 +201,7 @@ struct Hamiltonian {
   SpmmTuning tuning;
   std::shared_ptr<VirtualOp> virt;  // set for the on-the-fly product (nothing stored)
   std::shared_ptr<TiledOp> tiled;   // block-tiled copy of the FP32 values (8-vector product)
+  std::shared_ptr<FactoredOp> fact; // factored form of the same operator (factored.h)
   std::vector<uint64_t> blocks;     // neutron-block starts (+ n) when built from a basis
   bool use_tiled = true;            // route 8-vector FP32 products through `tiled` when present
   cudaStream_t stream = nullptr;

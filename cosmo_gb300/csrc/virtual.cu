@@ -26,6 +26,8 @@
 
 #include "bulk.h"
 #include "dfloat.h"
+#include "factored.h"
+#include "hostop.h"
 #include "tiled.h"
 #include "virtual.h"
 
@@ -35,62 +37,6 @@ namespace {
 
 constexpr double kDropV = 1e-14;
 constexpr int kVirtualSmemHead = 128;  // three mbarriers; keeps the staging buffers 128-byte aligned
-
-inline int popc(uint64_t x) { return __builtin_popcountll(x); }
-inline uint64_t below_h(int b) { return b >= 64 ? ~0ull : (1ull << b) - 1ull; }
-// global occupation words (neutron s.p. states from bit 0, protons above) of
-// up to 128 s.p. states, host only
-using G = unsigned __int128;
-inline int popg(G x) { return __builtin_popcountll(uint64_t(x)) + __builtin_popcountll(uint64_t(x >> 64)); }
-inline G below_g(int b) { return b >= 128 ? ~G(0) : ((G(1) << b) - 1); }
-inline G gbit(int b) { return G(1) << b; }
-inline int ctzg(G x) {
-  const uint64_t lo = uint64_t(x);
-  return lo ? __builtin_ctzll(lo) : 64 + __builtin_ctzll(uint64_t(x >> 64));
-}
-
-struct HostOp {
-  int ns = 0, np_pairs = 0;
-  std::vector<double> e1;      // ns x ns
-  std::vector<double> v2;      // npairs x npairs
-  std::vector<int32_t> pidx;   // ns x ns
-  double V(int a, int b, int c, int d) const {  // a < b, c < d
-    return v2[size_t(pidx[a * ns + b]) * np_pairs + pidx[c * ns + d]];
-  }
-  // forward two-body term (b0 < b1 annihilated, b2 < b3 created) on S0
-  double term2(G S0, int b0, int b1, int b2, int b3) const {
-    double v = V(b0, b1, b2, b3);
-    int p = popg(S0 & below_g(b0)) + popg(S0 & below_g(b1)) - 1;
-    G I = S0 & ~(gbit(b0) | gbit(b1));
-    p += popg(I & below_g(b2)) + popg(I & below_g(b3));
-    return (p & 1) ? -v : v;
-  }
-  double term1(G S0, int x, int y) const {
-    double v = e1[x * ns + y];
-    int p = popg(S0 & below_g(x)) + popg((S0 & ~gbit(x)) & below_g(y));
-    return (p & 1) ? -v : v;
-  }
-};
-
-HostOp host_operator(const System& sys, const Operator& op) {
-  HostOp h;
-  const int ns = int(sys.sps.size());
-  h.ns = ns;
-  h.pidx.assign(ns * ns, -1);
-  int np = 0;
-  for (int a = 0; a < ns; ++a)
-    for (int b = a + 1; b < ns; ++b) h.pidx[a * ns + b] = np++;
-  h.np_pairs = np;
-  h.e1.assign(ns * ns, 0.0);
-  for (auto& kv : op.one) h.e1[kv.first[0] * ns + kv.first[1]] = kv.second;
-  h.v2.assign(size_t(std::max(np, 1)) * std::max(np, 1), 0.0);
-  for (auto& kv : op.two) {
-    const Key4& k = kv.first;
-    if (k[0] >= k[1] || k[2] >= k[3]) continue;  // cannot act on a determinant
-    h.v2[size_t(h.pidx[k[0] * ns + k[1]]) * np + h.pidx[k[2] * ns + k[3]]] = kv.second;
-  }
-  return h;
-}
 
 // one-body move x -> y inside a species mask: phase parity of the other
 // occupied orbitals strictly between (the same from either end)
@@ -645,26 +591,34 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
   if (m < 1) throw Error(CG_ERR_ARG, "m must be >= 1");
   if (ldx < m || ldy < m) throw Error(CG_ERR_ARG, "leading dimension smaller than the vector count");
   const uint64_t n = h.n;
+  // n packed rows of 32 bytes in every precision, kept with the handle
+  DBuf<unsigned char>& pack = h.virt->pack;
+  if (n && !pack.p) pack.alloc(n * 32);
   if (precision == CG_PREC_FP32) {
-    DBuf<float> w(std::max<uint64_t>(n * kVirtualVB32, 1));
+    float* w = reinterpret_cast<float*>(pack.p);
+    const float* xf = static_cast<const float*>(x);
     for (int c0 = 0; c0 < m; c0 += kVirtualVB32) {
       const int mc = std::min(kVirtualVB32, m - c0);
-      virtual_pack_f32(n, static_cast<const float*>(x), ldx, c0, mc, w.p, s);
-      virtual_product_f32(h, w.p, static_cast<float*>(y) + c0, ldy, mc, s);
+      // rows that are packed already are taken as they are
+      const bool packed = mc == kVirtualVB32 && ldx == kVirtualVB32 && reinterpret_cast<uintptr_t>(x) % 32 == 0;
+      if (!packed) virtual_pack_f32(n, xf, ldx, c0, mc, w, s);
+      virtual_product_f32(h, packed ? xf : w, static_cast<float*>(y) + c0, ldy, mc, s);
     }
   } else if (precision == CG_PREC_REFINE) {
-    DBuf<float> w(std::max<uint64_t>(n * 8, 1));
+    float* w = reinterpret_cast<float*>(pack.p);
     for (int c0 = 0; c0 < m; c0 += 4) {
       const int mc = std::min(4, m - c0);
-      virtual_pack_df(n, static_cast<const double*>(x), ldx, c0, mc, w.p, s);
-      virtual_product_df(h, w.p, static_cast<double*>(y) + c0, ldy, mc, s);
+      virtual_pack_df(n, static_cast<const double*>(x), ldx, c0, mc, w, s);
+      virtual_product_df(h, w, static_cast<double*>(y) + c0, ldy, mc, s);
     }
   } else if (precision == CG_PREC_FP64) {
-    DBuf<double> w(std::max<uint64_t>(n * kVirtualVB64, 1));
+    double* w = reinterpret_cast<double*>(pack.p);
+    const double* xd = static_cast<const double*>(x);
     for (int c0 = 0; c0 < m; c0 += kVirtualVB64) {
       const int mc = std::min(kVirtualVB64, m - c0);
-      virtual_pack_f64(n, static_cast<const double*>(x), ldx, c0, mc, w.p, s);
-      virtual_product_f64(h, w.p, static_cast<double*>(y) + c0, ldy, mc, s);
+      const bool packed = mc == kVirtualVB64 && ldx == kVirtualVB64 && reinterpret_cast<uintptr_t>(x) % 32 == 0;
+      if (!packed) virtual_pack_f64(n, xd, ldx, c0, mc, w, s);
+      virtual_product_f64(h, packed ? xd : w, static_cast<double*>(y) + c0, ldy, mc, s);
     }
   } else {
     throw Error(CG_ERR_ARG, "unknown precision");
@@ -672,6 +626,7 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
 }
 
 void virtual_product_f32(const Hamiltonian& h, const float* x, float* y, int ldy, int m, cudaStream_t s) {
+  if (h.fact) return factored_product_f32(*h.fact, x, y, ldy, m, s);
   VTab<float> tb{h.virt->Wf.p, h.virt->Unf.p, h.virt->Upf.p, h.virt->sl_cf.p, h.virt->pp_hf.p};
   virtual_product<float, kVirtualVB32>(h, x, y, ldy, m, tb, tb, s);
 }
@@ -711,7 +666,7 @@ void virtual_pack_df(uint64_t n, const double* x, int ld, int c0, int m, float* 
 
 uint64_t Hamiltonian::device_bytes() const {
   return rowptr.bytes() + col.bytes() + val64.bytes() + hi.bytes() + lo.bytes() + diag.bytes() +
-         (virt ? virt->bytes() : 0) + (tiled ? tiled->bytes() : 0);
+         (virt ? virt->bytes() : 0) + (fact ? fact->bytes() : 0) + (tiled ? tiled->bytes() : 0);
 }
 
 // ------------------------------------------------------------------- build
@@ -1191,6 +1146,13 @@ void virtual_build(const System& sys, const Operator& op, const Basis& b, int pr
   }
   CG_CUDA(cudaStreamSynchronize(s));
   v.err.alloc(1);
+  // FP32 products: the factored form where it is estimated faster than k_virtual
+  // (40 us of launch and error read-back + 3.6 us per million elements for 8
+  // vectors, within 20 % from sd 4 + 4 to fp 4 + 4).  8 vectors, factored /
+  // k_virtual: fp 4 + 4 1.40 / 4.34 ms, fp 5 + 3 1.02 / 3.75, fp 3 + 3 0.07 / 0.26,
+  // sd 3 + 3 15 / 49 us; near half filling most pairs of a core are blocked and
+  // k_virtual stays (sd 6 + 6 172 / 129 us, sd 8 + 8 149 / 67).
+  h.fact = factored_build(sys, op, b, 40 + 3.6e-6 * double(conn), s);
   h.virt = vp;
   h.nnz = conn;
   h.nnz_upper = 0;

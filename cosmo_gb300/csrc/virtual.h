@@ -82,6 +82,7 @@ struct VirtualOp {
   DBuf<uint16_t> lmap;                              // per list: class rank -> list rank
   DBuf<uint32_t> lmap_off, lmap_len;                // lists: first entry, entries (16-byte multiples)
   mutable DBuf<int> err;                            // staged-copy timeout flag
+  mutable DBuf<unsigned char> pack;                 // packed operand of virtual_launch (first use)
   uint64_t bytes() const {
     return bstart.bytes() + blen.bytes() + bclass.bytes() + bmask.bytes() + order.bytes() + cstart.bytes() +
            cmask.bytes() + nt_off.bytes() + nt.bytes() + nn_off.bytes() + nn2.bytes() + cslice.bytes() +
@@ -89,11 +90,12 @@ struct VirtualOp {
            pp_h.bytes() + pp_hf.bytes() + W.bytes() + Un.bytes() + Up.bytes() +
            Wf.bytes() + Unf.bytes() + Upf.bytes() + Wl.bytes() + Unl.bytes() + Upl.bytes() + sl_cl.bytes() +
            pp_hl.bytes() + gcr.bytes() + lmap.bytes() + lmap_off.bytes() + lmap_len.bytes() + bmask64.bytes() +
-           cmask64.bytes();
+           cmask64.bytes() + pack.bytes();
   }
 };
 
-// Tables + diagonal for the on-the-fly product (h.diag filled, h.virt set).
+// Tables + diagonal for the on-the-fly product (h.diag filled, h.virt set, and
+// h.fact where the factored form (factored.h) serves its FP32 products).
 void virtual_build(const System& sys, const Operator& op, const Basis& b, int precision, Hamiltonian& h);
 
 // y[i*ldy + k] = (H x)[i][k], k < m, from x packed as n rows of kVirtualVB<T>
@@ -109,7 +111,7 @@ constexpr int kVirtualVB32 = 8, kVirtualVB64 = 4;
 // pack columns c0 .. c0+m of a row-interleaved block into the product's layout
 void virtual_pack_f32(uint64_t n, const float* x, int ld, int c0, int m, float* w, cudaStream_t s);
 void virtual_pack_f64(uint64_t n, const double* x, int ld, int c0, int m, double* w, cudaStream_t s);
-// general row-interleaved operands (any m, any ld); allocates its packing buffer
+// general row-interleaved operands (any m, any ld), packed in a buffer of the handle
 void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx, void* y, int ldy, int m,
                     cudaStream_t s);
 
