@@ -28,7 +28,7 @@ LIB_PATH = os.path.join(_HERE, "libcosmo_gb300.so")
 CG_OK = 0
 CG_ERR_ARG = -1
 CG_PREC_FP64, CG_PREC_FP32, CG_PREC_REFINE = 0, 1, 2
-CG_FORMAT_ROWS, CG_FORMAT_TILED = 0, 1
+CG_FORMAT_ROWS, CG_FORMAT_TILED, CG_FORMAT_FACTORED = 0, 1, 2
 STATUS_NAMES = {0: "CG_OK", -1: "CG_ERR_ARG", -2: "CG_ERR_IO", -3: "CG_ERR_PARSE", -4: "CG_ERR_CUDA",
                 -5: "CG_ERR_NOMEM", -6: "CG_ERR_UNSUPPORTED", -7: "CG_ERR_NOT_CONVERGED",
                 -8: "CG_ERR_TIMEOUT", -9: "CG_ERR_NO_DEVICE", -10: "CG_ERR_INTERNAL"}
@@ -156,6 +156,7 @@ _SIGS = {
     "cg_spmm_get_tuning": (C.c_int32, [_P, C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "cg_spmm_set_format": (C.c_int32, [_P, C.c_int32]),
     "cg_spmm_get_format": (C.c_int32, [_P, _P]),
+    "cg_spmm_format_in_use": (C.c_int32, [_P, C.POINTER(C.c_int32)]),
     "cg_spmm_set_tiled_shape": (C.c_int32, [_P, C.c_int32, C.c_int32]),
     "cg_davidson_defaults": (None, [C.POINTER(DavidsonParams), C.c_int32]),
     "cg_davidson": (C.c_int32, [_P, C.POINTER(DavidsonParams), _P, C.c_int32, _P, _P, _P, _P,
@@ -555,9 +556,16 @@ class Hamiltonian:
                 w, c = db[key]["warps"], db[key]["ctas_per_sm"]
                 _check(lib().cg_spmm_set_tuning(self._h, w, c))
                 fmt = db[key].get("format", CG_FORMAT_ROWS)
-                if fmt == CG_FORMAT_TILED and not self.format()[1]:
+                if fmt == CG_FORMAT_FACTORED:
+                    try:
+                        self.set_format(fmt)
+                    except CosmoError:  # no factored form of this matrix here
+                        fmt = CG_FORMAT_ROWS
+                elif fmt == CG_FORMAT_ROWS and self.format_in_use() == CG_FORMAT_FACTORED:
+                    self.set_format(fmt)
+                elif fmt == CG_FORMAT_TILED and not self.format()[1]:
                     fmt = CG_FORMAT_ROWS
-                if self.format()[1]:
+                elif self.format()[1]:
                     self.set_format(fmt)
                     if "tiled_shape" in db[key]:
                         self.set_tiled_shape(*db[key]["tiled_shape"])
@@ -569,7 +577,7 @@ class Hamiltonian:
         _check(lib().cg_spmm_autotune(self._h, nvec, reps, C.byref(cap), _ptr(w), _ptr(c), _ptr(ms)))
         k = int(cap.value)
         bw, bc, _ = self.tuning()
-        fmt = self.format()[0]
+        fmt = self.format_in_use()
         res = {"warps": bw, "ctas_per_sm": bc, "format": fmt, "cached": False,
                "candidates": [(int(w[i]), int(c[i]), float(ms[i])) for i in range(k)]}
         if cache:
@@ -578,7 +586,7 @@ class Hamiltonian:
                 with open(cache) as f:
                     db = json.load(f)
             db[key] = {"warps": bw, "ctas_per_sm": bc, "format": fmt, "ms": float(min(ms[:k]))}
-            fi = self.format_info()
+            fi = self.format_info() if fmt != CG_FORMAT_FACTORED else {"tiled_available": False}
             if fi["tiled_available"]:
                 db[key]["tiled_shape"] = [fi["slices_per_warp"], fi["stages"]]
             with open(cache, "w") as f:
@@ -591,9 +599,15 @@ class Hamiltonian:
         return int(w.value), int(c.value), bool(t.value)
 
     def set_format(self, fmt: int) -> None:
-        """Storage the FP32 product of up to 8 vectors reads: CG_FORMAT_ROWS
-        (row-wise) or CG_FORMAT_TILED (neutron-block tiles)."""
+        """What the FP32 product of up to 8 vectors reads: CG_FORMAT_ROWS
+        (row-wise), CG_FORMAT_TILED (neutron-block tiles) or
+        CG_FORMAT_FACTORED (two-particle cores)."""
         _check(lib().cg_spmm_set_format(self._h, fmt))
+
+    def format_in_use(self) -> int:
+        f = C.c_int32()
+        _check(lib().cg_spmm_format_in_use(self._h, C.byref(f)))
+        return int(f.value)
 
     def format(self):
         """(format in use, tiled copy present, tiled entries incl. padding)."""

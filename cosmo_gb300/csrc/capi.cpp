@@ -723,10 +723,24 @@ cg_status cg_spmm_get_tuning(const cg_hamiltonian* h, int32_t* warps, int32_t* c
   });
 }
 
+namespace {
+// A large matrix whose products run factored gets its block-tiled copy when it
+// is first asked about.
+void tiled_on_demand(const cg_hamiltonian* ch) {
+  cg::Hamiltonian& h = const_cast<cg_hamiltonian*>(ch)->h;
+  if (h.tiled || h.virt || !h.fact || h.nnz < cg::kTiledMinEntries) return;
+  CG_CUDA(cudaSetDevice(h.device));
+  cg::tiled_build(h, h.blocks);
+}
+}  // namespace
+
 cg_status cg_spmm_set_format(cg_hamiltonian* h, int32_t format) {
   return guard([&] {
     CG_NOT_NULL(h);
-    if (format != CG_FORMAT_ROWS && format != CG_FORMAT_TILED) throw cg::Error(CG_ERR_ARG, "unknown SpMM format");
+    if (format != CG_FORMAT_ROWS && format != CG_FORMAT_TILED && format != CG_FORMAT_FACTORED)
+      throw cg::Error(CG_ERR_ARG, "unknown SpMM format");
+    if (format == CG_FORMAT_FACTORED && (!h->h.fact || h->h.virt))
+      throw cg::Error(CG_ERR_UNSUPPORTED, "no factored form of this matrix");
     if (format == CG_FORMAT_TILED && !h->h.tiled && !h->h.virt && h->h.precision == CG_PREC_FP32 &&
         !h->h.blocks.empty()) {
       CG_CUDA(cudaSetDevice(h->h.device));
@@ -735,13 +749,14 @@ cg_status cg_spmm_set_format(cg_hamiltonian* h, int32_t format) {
     if (format == CG_FORMAT_TILED && !h->h.tiled)
       throw cg::Error(CG_ERR_UNSUPPORTED,
                       "no block-tiled copy (needs an FP32 matrix built from a basis, blocks <= 1536 rows)");
-    h->h.use_tiled = format == CG_FORMAT_TILED;
+    h->h.format = format;
   });
 }
 
 cg_status cg_spmm_set_tiled_shape(cg_hamiltonian* h, int32_t slices_per_warp, int32_t stages) {
   return guard([&] {
     CG_NOT_NULL(h);
+    tiled_on_demand(h);
     cg::TiledOp* t = h->h.tiled.get();
     if (!t) throw cg::Error(CG_ERR_UNSUPPORTED, "no block-tiled copy");
     if (slices_per_warp < 1 || slices_per_warp > 4) throw cg::Error(CG_ERR_ARG, "slices per warp must be 1..4");
@@ -755,13 +770,27 @@ cg_status cg_spmm_set_tiled_shape(cg_hamiltonian* h, int32_t slices_per_warp, in
   });
 }
 
+static int32_t format_in_use(const cg::Hamiltonian& h) {
+  if (h.virt) return CG_FORMAT_ROWS;
+  return h.use_fact() ? CG_FORMAT_FACTORED : h.use_tiled() ? CG_FORMAT_TILED : CG_FORMAT_ROWS;
+}
+
+cg_status cg_spmm_format_in_use(const cg_hamiltonian* h, int32_t* format) {
+  return guard([&] {
+    CG_NOT_NULL(h);
+    CG_NOT_NULL(format);
+    *format = format_in_use(h->h);
+  });
+}
+
 cg_status cg_spmm_get_format(const cg_hamiltonian* h, cg_spmm_format_info* info) {
   return guard([&] {
     CG_NOT_NULL(h);
     CG_NOT_NULL(info);
     *info = cg_spmm_format_info{};
+    tiled_on_demand(h);
     const cg::TiledOp* t = h->h.tiled.get();
-    info->format = t && h->h.use_tiled ? CG_FORMAT_TILED : CG_FORMAT_ROWS;
+    info->format = format_in_use(h->h);
     info->tiled_available = t != nullptr;
     if (t) {
       info->warps = t->warps;

@@ -1116,12 +1116,16 @@ struct Engine {
     } else if constexpr (sizeof(T) == 4) {
       if (cfg.spmm_prec == CG_PREC_FP32) {
         if (!stage.p) stage.alloc(n * 16);
-        int pad = m <= 8 ? 8 : 16;
-        k_stage_block<<<blocks_for(n * pad), 256, 0, s>>>(n, reinterpret_cast<const float*>(B.p), L, c0, m,
-                                                            stage.p, pad);
-        CG_CUDA(cudaGetLastError());
-    count_launch();
-        spmm_f32_padded(H, stage.p, pad, reinterpret_cast<float*>(AB.p) + c0, L, m, s);
+        // up to 16 vectors a pass row-wise, 8 through the factored form
+        const int most = H.use_fact() ? 8 : 16;
+        for (int c = 0; c < m; c += most) {
+          const int mc = std::min(most, m - c), pad = mc <= 8 ? 8 : 16;
+          k_stage_block<<<blocks_for(n * pad), 256, 0, s>>>(n, reinterpret_cast<const float*>(B.p), L, c0 + c, mc,
+                                                              stage.p, pad);
+          CG_CUDA(cudaGetLastError());
+          count_launch();
+          spmm_f32_padded(H, stage.p, pad, reinterpret_cast<float*>(AB.p) + c0 + c, L, mc, s);
+        }
       } else {
         spmm_launch(H, cfg.spmm_prec, B.p + c0, L, AB.p + c0, L, m, s);
       }

@@ -203,7 +203,9 @@ struct Hamiltonian {
   std::shared_ptr<TiledOp> tiled;   // block-tiled copy of the FP32 values (8-vector product)
   std::shared_ptr<FactoredOp> fact; // factored form of the same operator (factored.h)
   std::vector<uint64_t> blocks;     // neutron-block starts (+ n) when built from a basis
-  bool use_tiled = true;            // route 8-vector FP32 products through `tiled` when present
+  int format = CG_FORMAT_TILED;     // what FP32 products of up to 8 vectors use, where it exists
+  bool use_fact() const { return fact && format == CG_FORMAT_FACTORED; }
+  bool use_tiled() const { return tiled && format == CG_FORMAT_TILED; }
   cudaStream_t stream = nullptr;
   ~Hamiltonian();
   uint64_t device_bytes() const;  // HBM held by the matrix (or the on-the-fly tables)
@@ -219,7 +221,8 @@ struct WideRows {
 };
 std::unique_ptr<WideRows> wide_rows(const System& sys, const Operator& op, const Basis& b, cudaStream_t s);
 
-// tiled_copy: also build the block-tiled copy of an FP32 matrix (tiled.h)
+// tiled_copy: also build the factored form (factored.h) of a large FP32 matrix or,
+// where that does not serve it, the block-tiled copy (tiled.h)
 void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, int precision, Hamiltonian& h,
                        bool tiled_copy = true);
 void hamiltonian_upper_rows(const Hamiltonian& h, uint64_t row0, uint64_t nrows, uint64_t* rowptr, uint32_t* cols,

@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "device.h"
+#include "factored.h"
 #include "tiled.h"
 #include "virtual.h"
 
@@ -486,10 +487,10 @@ void spmm_host(const Hamiltonian& h, int precision, const double* x, double* y, 
 }
 
 // Autotuner: time every candidate launch shape of the row-wise FP32 product on
-// this matrix and, for up to 8 vectors, the block-tiled product (CUDA events
-// on the handle's stream, median of `reps`); keep the fastest in h.tuning /
-// h.use_tiled.  Returns the per-candidate times (the tiled candidate carries
-// ctas_per_sm = 0).  Shapes with fewer than 16 resident warps per SM are not
+// this matrix and, for up to 8 vectors, the factored and the block-tiled
+// product where they exist (CUDA events on the handle's stream, median of
+// `reps`); keep the fastest in h.tuning / h.format.  Returns the per-candidate
+// times (the tiled candidate carries ctas_per_sm = 0, the factored one -1).  Shapes with fewer than 16 resident warps per SM are not
 // tried (the gathers of the row-wise product need more in flight; they were
 // 2-6x slower than the best on every matrix measured), and a candidate whose
 // warm-up launch takes more than twice the best median so far is not
@@ -529,8 +530,8 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
   std::vector<SpmmCandidate> out;
   const SpmmTuning keep = h.tuning;
   SpmmTuning bt = keep;
-  bool tiled_best = false;
-  h.use_tiled = false;
+  int best_format = CG_FORMAT_ROWS;
+  h.format = CG_FORMAT_ROWS;
   for (int w : {4, 8, 16, 32})
     for (int c : {1, 2, 4, 8}) {
       if (w * c > 64 || w * c < 16) continue;  // 16..64 resident warps per SM
@@ -545,7 +546,7 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
     TiledOp& t = *h.tiled;
     int brps = t.rps, bst = t.stages;
     float tbest = 1e30f;
-    h.use_tiled = true;
+    h.format = CG_FORMAT_TILED;
     for (int rps : {1, 2, 3})
       for (int st : {2, 3, 4, 6}) {
         if ((t.smax + rps - 1) / rps > 31) continue;  // at most 31 consumer warps
@@ -561,11 +562,17 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
     t.stages = bst;
     const int bw = t.warps;
     out.push_back({bw, 0, tbest});
-    if (tbest < best) { best = tbest; tiled_best = true; }
+    if (tbest < best) { best = tbest; best_format = CG_FORMAT_TILED; }
+  }
+  if (h.fact && m <= 8) {
+    h.format = CG_FORMAT_FACTORED;
+    const float med = time_once();
+    out.push_back({0, -1, med});
+    if (med < best) { best = med; best_format = CG_FORMAT_FACTORED; }
   }
   h.tuning = bt;
   h.tuning.tuned = true;
-  h.use_tiled = tiled_best;
+  h.format = best_format;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   return out;
@@ -721,7 +728,8 @@ void spmm_f32_padded(const Hamiltonian& h, const float* x, int ldx, float* y, in
   if (h.precision != CG_PREC_FP32) throw Error(CG_ERR_ARG, "FP32 product needs an FP32 matrix");
   if (m < 1 || m > 16) throw Error(CG_ERR_ARG, "padded FP32 SpMM takes 1..16 vectors");
   if (reinterpret_cast<uintptr_t>(x) % 32 || ldx % 8) throw Error(CG_ERR_ARG, "padded FP32 SpMM needs 32-byte rows");
-  if (m <= 8 && ldx == 8 && h.tiled && h.use_tiled) return tiled_product(h, x, y, ldy, m, s);
+  if (m <= 8 && ldx == 8 && h.use_fact()) return factored_product_f32(*h.fact, x, y, ldy, m, s);
+  if (m <= 8 && ldx == 8 && h.use_tiled()) return tiled_product(h, x, y, ldy, m, s);
   if (m <= 8) {
     if (ldx < 8) throw Error(CG_ERR_ARG, "ldx < 8");
     run_wide<8>(h, x, ldx, y, ldy, m, s);
@@ -743,7 +751,9 @@ void spmm_launch(const Hamiltonian& h, int precision, const void* x, int ldx, vo
       break;
     case CG_PREC_FP32:
       if (h.precision != CG_PREC_FP32) throw Error(CG_ERR_ARG, "FP32 product needs an FP32 matrix");
-      if (m <= 8 && ldx == 8 && h.tiled && h.use_tiled && reinterpret_cast<uintptr_t>(x) % 16 == 0)
+      if (m <= 8 && ldx == 8 && h.use_fact() && reinterpret_cast<uintptr_t>(x) % 32 == 0)
+        return factored_product_f32(*h.fact, static_cast<const float*>(x), static_cast<float*>(y), ldy, m, s);
+      if (m <= 8 && ldx == 8 && h.use_tiled() && reinterpret_cast<uintptr_t>(x) % 16 == 0)
         return tiled_product(h, static_cast<const float*>(x), static_cast<float*>(y), ldy, m, s);
       dispatch_nv<CG_PREC_FP32>(m, h, h.hi.p, x, ldx, y, ldy, s);
       break;

@@ -238,19 +238,26 @@ cg_status cg_gather_ceiling(uint64_t rows, int32_t share, double* gathers_per_se
 /* Set (e.g. from a cached tuning) or read the launch shape of the FP32 product. */
 cg_status cg_spmm_set_tuning(cg_hamiltonian* h, int32_t warps, int32_t ctas_per_sm);
 cg_status cg_spmm_get_tuning(const cg_hamiltonian* h, int32_t* warps, int32_t* ctas_per_sm, int32_t* tuned);
-/* Storage the FP32 product of up to 8 vectors reads.  An FP32 matrix built
- * from a basis also holds a block-tiled copy: tiles = (neutron block, neutron
- * block) pairs, 16-bit in-tile columns, x of the column block staged in shared
- * memory per tile.  The reference's counterpart is its fixed CSB blocking
+/* What the FP32 product of up to 8 vectors (row stride 8) reads: the stored
+ * rows, a block-tiled copy, or the factored form of the same operator.
+ * Factored: H applied through the determinants with two particles taken out,
+ * small dense matrices per core instead of the stored elements; an FP32 matrix
+ * of 2^25 stored entries or more, built from an untruncated basis, uses it by
+ * default where it is estimated faster.  Block-tiled copy of an FP32 matrix
+ * built from a basis: tiles = (neutron block, neutron block) pairs, 16-bit
+ * in-tile columns, x of the column block staged in shared memory per tile.  The reference's counterpart is its fixed CSB blocking
  * (PPMatrix2CSBBlk, include/sm/PPMatrix.cxx:571-656); the choice of format has
- * no counterpart there.  The copy is built with the matrix from 2^26 stored
- * entries up, and on request (cg_spmm_set_format(h, CG_FORMAT_TILED)) below.
- * cg_spmm_autotune picks the faster format when the copy exists (its tiled
- * candidate is reported with ctas_per_sm = 0). */
+ * no counterpart there.  From 2^26 stored entries up the copy is built with the
+ * matrix, or when first asked about (cg_spmm_get_format, cg_spmm_set_format,
+ * cg_spmm_set_tiled_shape) if the matrix uses its factored form; below, on
+ * request (cg_spmm_set_format(h, CG_FORMAT_TILED)).  cg_spmm_autotune picks the
+ * fastest of the formats that exist (its tiled candidate is reported with
+ * ctas_per_sm = 0, the factored one with -1). */
 #define CG_FORMAT_ROWS 0
 #define CG_FORMAT_TILED 1
+#define CG_FORMAT_FACTORED 2
 typedef struct {
-  int32_t format;          /* CG_FORMAT_ROWS or CG_FORMAT_TILED (in use for <= 8 FP32 vectors) */
+  int32_t format;          /* CG_FORMAT_* in use for <= 8 FP32 vectors */
   int32_t tiled_available; /* the block-tiled copy exists */
   int32_t warps, stages;   /* tiled product: consumer warps per CTA, ring slots */
   int32_t slices_per_warp; /* tiled product: 32-row slices per consumer warp */
@@ -264,6 +271,8 @@ typedef struct {
 } cg_spmm_format_info;
 cg_status cg_spmm_set_format(cg_hamiltonian* h, int32_t format);
 cg_status cg_spmm_get_format(const cg_hamiltonian* h, cg_spmm_format_info* info);
+/* The format in use alone (CG_FORMAT_*); builds nothing. */
+cg_status cg_spmm_format_in_use(const cg_hamiltonian* h, int32_t* format);
 /* Launch shape of the tiled product (e.g. from a cached tuning): 32-row slices
  * per consumer warp (1..4, at most 31 consumer warps) and ring slots (2..7,
  * within 227 KB of shared memory). */
