@@ -69,15 +69,59 @@ __device__ __forceinline__ void load_vec(const double* __restrict__ p, double (&
   }
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 __device__ __forceinline__ float warp_sumf(float v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// FP64 and REFINE products: half a warp per row.  They are bound by the FP64
+// pipe (2 multiply-adds per clock and SM, an instruction costs the same for 1
+// or 32 active lanes), so the row sums go through a reduce-scatter over the 16
+// lanes (NV = 4: 5 additions a pair of rows instead of 20 a row) and two rows
+// share an instruction, which also halves the unused lanes of the last step
+// of a row.  sd 6+6, 4 vectors: 292 -> 186 us (the pipe alone 162).
+template <int NV, int MODE, int VW>
+__device__ __forceinline__ void rows_f64(uint64_t n, const uint64_t* __restrict__ rowptr,
+                                         const uint32_t* __restrict__ col, const void* __restrict__ vals,
+                                         const float* __restrict__ lo, const double* __restrict__ x, int ldx,
+                                         double* __restrict__ y, int ldy, uint64_t r0, uint64_t r1) {
+  constexpr int P = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 4 : NV <= 8 ? 8 : 16;
+  constexpr int kGroup = 16 / P;  // lanes sharing a component after the reduce-scatter
+  const int lane = threadIdx.x & 31, half = lane >> 4, l = lane & 15, warp = threadIdx.x >> 5;
+  for (uint64_t base = r0 + warp * 2; base < r1; base += kWarpsPerCta * 2) {  // warp-uniform
+    const uint64_t row = base + half;
+    const bool live = row < r1;
+    const uint64_t b = live ? __ldg(rowptr + row) : 0, e = live ? __ldg(rowptr + row + 1) : 0;
+    double acc[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) acc[k] = 0.0;
+    for (uint64_t p = b + l; p < e; p += 16) {
+      const uint32_t c = __ldcs(col + p);
+      double h;
+      if constexpr (MODE == CG_PREC_FP64) h = __ldcs(static_cast<const double*>(vals) + p);
+      else h = double(__ldcs(static_cast<const float*>(vals) + p)) + double(__ldcs(lo + p));
+      double xx[NV];
+      load_vec<NV, VW>(x + uint64_t(c) * ldx, xx);
+#pragma unroll
+      for (int k = 0; k < NV; ++k) acc[k] = fma(h, xx[k], acc[k]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 8, c = P; c > 1; o >>= 1, c >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < c / 2; ++k) {
+        const double send = up ? acc[k] : acc[c / 2 + k];
+        const double keep = up ? acc[c / 2 + k] : acc[k];
+        acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+#pragma unroll
+    for (int o = kGroup >> 1; o; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    const int k = l / kGroup;
+    if (live && l % kGroup == 0 && k < NV) y[row * uint64_t(ldy) + k] = acc[0];
+  }
 }
 
 // Each CTA owns rows [r0, r1); its warps take rows r0 + w, r0 + w + 8, ...
@@ -88,17 +132,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_spmm(uint64_t n, const ui
                                                             const float* __restrict__ lo, const void* __restrict__ xv,
                                                             int ldx, void* __restrict__ yv, int ldy,
                                                             uint64_t rows_per_cta) {
-  using XT = typename std::conditional<MODE == CG_PREC_FP32, float, double>::type;
-  const XT* x = static_cast<const XT*>(xv);
-  XT* y = static_cast<XT*>(yv);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t r0 = uint64_t(blockIdx.x) * rows_per_cta;
   const uint64_t r1 = min(n, r0 + rows_per_cta);
-  for (uint64_t row = r0 + warp; row < r1; row += kWarpsPerCta) {
-    const uint64_t b = __ldg(rowptr + row), e = __ldg(rowptr + row + 1);
-    double tot[NV];
-    if constexpr (MODE == CG_PREC_FP32) {
-      const float* hv = static_cast<const float*>(vals);
+  if constexpr (MODE != CG_PREC_FP32) {
+    rows_f64<NV, MODE, VW>(n, rowptr, col, vals, lo, static_cast<const double*>(xv), ldx, static_cast<double*>(yv),
+                           ldy, r0, r1);
+  } else {
+    const float* x = static_cast<const float*>(xv);
+    float* y = static_cast<float*>(yv);
+    const float* hv = static_cast<const float*>(vals);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t row = r0 + warp; row < r1; row += kWarpsPerCta) {
+      const uint64_t b = __ldg(rowptr + row), e = __ldg(rowptr + row + 1);
       float acc[NV];
 #pragma unroll
       for (int k = 0; k < NV; ++k) acc[k] = 0.f;
@@ -112,31 +157,14 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_spmm(uint64_t n, const ui
       }
       // cross-lane sum in FP32: on GB300 an FP64 warp reduction per row costs
       // more FP64-pipe time than the whole row's memory traffic
+      float mine = 0.f;
 #pragma unroll
-      for (int k = 0; k < NV; ++k) tot[k] = double(warp_sumf(acc[k]));
-    } else {
-      double acc[NV];
-#pragma unroll
-      for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-      for (uint64_t p = b + lane; p < e; p += 32) {
-        const uint32_t c = __ldcs(col + p);
-        double h;
-        if constexpr (MODE == CG_PREC_FP64) h = __ldcs(static_cast<const double*>(vals) + p);
-        else h = double(__ldcs(static_cast<const float*>(vals) + p)) + double(__ldcs(lo + p));
-        double xx[NV];
-        load_vec<NV, VW>(x + uint64_t(c) * ldx, xx);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) acc[k] = fma(h, xx[k], acc[k]);
+      for (int k = 0; k < NV; ++k) {
+        const float t = warp_sumf(acc[k]);
+        if (lane == k) mine = t;  // lane k writes component k
       }
-#pragma unroll
-      for (int k = 0; k < NV; ++k) tot[k] = warp_sum(acc[k]);
+      if (lane < NV) y[row * uint64_t(ldy) + lane] = mine;
     }
-    // lane k writes component k (all lanes hold every total after the xor-reduction)
-    double mine = 0.0;
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-      if (lane == k) mine = tot[k];
-    if (lane < NV) y[row * uint64_t(ldy) + lane] = XT(mine);
   }
 }
 
@@ -236,8 +264,9 @@ void run_kernel(const Hamiltonian& h, const void* vals, const void* x, int ldx, 
   CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm<NV, MODE, VW>, kWarpsPerCta * 32, 0));
   uint64_t ctas = uint64_t(nsm) * std::max(per_sm, 1) * 4;
   uint64_t rpc = (h.n + ctas - 1) / ctas;
-  rpc = (rpc + kWarpsPerCta - 1) / kWarpsPerCta * kWarpsPerCta;
-  if (rpc == 0) rpc = kWarpsPerCta;
+  constexpr int kStep = MODE == CG_PREC_FP32 ? kWarpsPerCta : 2 * kWarpsPerCta;  // rows a CTA takes at a time
+  rpc = (rpc + kStep - 1) / kStep * kStep;
+  if (rpc == 0) rpc = kStep;
   unsigned grid = unsigned((h.n + rpc - 1) / rpc);
   if (grid == 0) return;
   k_spmm<NV, MODE, VW><<<grid, kWarpsPerCta * 32, 0, s>>>(h.n, h.rowptr.p, h.col.p, vals, h.lo.p, x, ldx, y, ldy,
@@ -673,7 +702,7 @@ void spmm_refine_df(const Hamiltonian& h, const double* x, int ldx, double* y, i
 
 // ---- allocation-free refinement product ------------------------------------
 // The double-float product stages each block of 8 columns of x as 16 floats per
-// row (8 high parts, then 8 low parts).  spmm_refine_static keeps that staging
+// row at most (8 high parts, then 8 low parts).  spmm_refine_static keeps that staging
 // area in the fixed device array below instead of a per-call allocation, for
 // callers that cannot allocate device memory: a host eigensolver that drives
 // the product while the stored matrix and its vector basis hold the device's
