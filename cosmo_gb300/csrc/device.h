@@ -202,6 +202,7 @@ struct Hamiltonian {
   std::shared_ptr<VirtualOp> virt;  // set for the on-the-fly product (nothing stored)
   std::shared_ptr<TiledOp> tiled;   // block-tiled copy of the FP32 values (8-vector product)
   std::shared_ptr<FactoredOp> fact; // factored form of the same operator (factored.h)
+  mutable DBuf<unsigned char> host_work;  // device buffers of host products (spmm_host)
   std::vector<uint64_t> blocks;     // neutron-block starts (+ n) when built from a basis
   int format = CG_FORMAT_TILED;     // what FP32 products of up to 8 vectors use, where it exists
   bool use_fact() const { return fact && format == CG_FORMAT_FACTORED; }

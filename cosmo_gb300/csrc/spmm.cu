@@ -309,11 +309,13 @@ __device__ __forceinline__ df32 df_add(df32 a, df32 b) {
   return quick_two_sum(s.hi, s.lo);
 }
 
-// Y = H X for 8 vectors in double-float.  X is staged as rows of 16 floats:
-// 8 hi parts then 8 lo parts (two sector-wide gathers per stored entry); the
-// matrix values are the stored (hi, lo) pair; Y is written as FP64.
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_spmm_df8(uint64_t n, const uint64_t* __restrict__ rowptr,
+// Y = H X for NV = 4 or 8 vectors in double-float.  X is staged as rows of 2 NV
+// floats: NV hi parts then NV lo parts (one or two sector-wide gathers per
+// stored entry); the matrix values are the stored (hi, lo) pair; Y is written
+// as FP64.  The FP32 pipe bounds it (about 17 operations an entry and vector), so
+// up to 4 vectors take the narrow form (sd 5+6: 182 -> 101 us).
+template <int NV, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_spmm_df(uint64_t n, const uint64_t* __restrict__ rowptr,
                                                          const uint32_t* __restrict__ col,
                                                          const float* __restrict__ vhi,
                                                          const float* __restrict__ vlo,
@@ -324,13 +326,13 @@ __global__ void __launch_bounds__(WARPS * 32) k_spmm_df8(uint64_t n, const uint6
   const uint64_t r1 = min(n, r0 + rows_per_cta);
   for (uint64_t row = r0 + warp; row < r1; row += WARPS) {
     const uint64_t b = __ldg(rowptr + row), e = __ldg(rowptr + row + 1);
-    df32 acc[8];
+    df32 acc[NV];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = {0.f, 0.f};
+    for (int k = 0; k < NV; ++k) acc[k] = {0.f, 0.f};
     uint64_t p = b + lane;
     for (; p + 32 < e; p += 64) {
       uint32_t c[2];
-      float hh[2], hl[2], xh[2][8], xl[2][8];
+      float hh[2], hl[2], xx[2][2 * NV];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         c[u] = __ldcs(col + p + 32 * u);
@@ -338,27 +340,36 @@ __global__ void __launch_bounds__(WARPS * 32) k_spmm_df8(uint64_t n, const uint6
         hl[u] = __ldcs(vlo + p + 32 * u);
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        ld8(x + uint64_t(c[u]) * 16, xh[u]);
-        ld8(x + uint64_t(c[u]) * 16 + 8, xl[u]);
-      }
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int g = 0; g < NV / 4; ++g) {
+          float t[8];
+          ld8(x + uint64_t(c[u]) * (2 * NV) + 8 * g, t);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) xx[u][8 * g + j] = t[j];
+        }
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) df_fma(acc[k], hh[u], hl[u], xh[u][k], xl[u][k]);
+        for (int k = 0; k < NV; ++k) df_fma(acc[k], hh[u], hl[u], xx[u][k], xx[u][NV + k]);
     }
     for (; p < e; p += 32) {
       const uint32_t c = __ldcs(col + p);
       const float hh = __ldcs(vhi + p), hl = __ldcs(vlo + p);
-      float xh[8], xl[8];
-      ld8(x + uint64_t(c) * 16, xh);
-      ld8(x + uint64_t(c) * 16 + 8, xl);
+      float xx[2 * NV];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) df_fma(acc[k], hh, hl, xh[k], xl[k]);
+      for (int g = 0; g < NV / 4; ++g) {
+        float t[8];
+        ld8(x + uint64_t(c) * (2 * NV) + 8 * g, t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xx[8 * g + j] = t[j];
+      }
+#pragma unroll
+      for (int k = 0; k < NV; ++k) df_fma(acc[k], hh, hl, xx[k], xx[NV + k]);
     }
-    // reduce-scatter across the warp (offsets 16, 8, 4), then offsets 2, 1
+    // reduce-scatter across the warp (offsets 16, 8 and, for 8 vectors, 4), then the rest
 #pragma unroll
-    for (int o = 16, cnt = 8; cnt > 1; o >>= 1, cnt >>= 1) {
+    for (int o = 16, cnt = NV; cnt > 1; o >>= 1, cnt >>= 1) {
       const bool up = lane & o;
 #pragma unroll
       for (int k = 0; k < cnt / 2; ++k) {
@@ -368,26 +379,51 @@ __global__ void __launch_bounds__(WARPS * 32) k_spmm_df8(uint64_t n, const uint6
         acc[k] = df_add(keep, got);
       }
     }
+    constexpr int kLanes = 32 / NV;  // lanes per vector
 #pragma unroll
-    for (int o = 2; o; o >>= 1) {
+    for (int o = kLanes >> 1; o; o >>= 1) {
       df32 got{__shfl_xor_sync(0xffffffffu, acc[0].hi, o), __shfl_xor_sync(0xffffffffu, acc[0].lo, o)};
       acc[0] = df_add(acc[0], got);
     }
-    const int vi = lane >> 2;
-    if ((lane & 3) == 0 && vi < m_out) y[row * uint64_t(ldy) + vi] = double(acc[0].hi) + double(acc[0].lo);
+    const int vi = lane / kLanes;
+    if (lane % kLanes == 0 && vi < m_out) y[row * uint64_t(ldy) + vi] = double(acc[0].hi) + double(acc[0].lo);
   }
 }
 
-// x (FP64, row-interleaved, m <= 8 columns) -> staging rows of 8 hi + 8 lo floats
+// x (FP64, row-interleaved, m <= NV columns) -> staging rows of NV hi + NV lo floats
+template <int NV>
 __global__ void k_stage_df(uint64_t n, const double* __restrict__ x, int ldx, int m, float* __restrict__ w) {
   uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (idx >= n * 8) return;
-  uint64_t i = idx >> 3;
-  int j = int(idx & 7);
+  if (idx >= n * NV) return;
+  uint64_t i = idx / NV;
+  int j = int(idx % NV);
   double v = j < m ? x[i * ldx + j] : 0.0;
   float h = float(v);
-  w[i * 16 + j] = h;
-  w[i * 16 + 8 + j] = float(v - double(h));
+  w[i * (2 * NV) + j] = h;
+  w[i * (2 * NV) + NV + j] = float(v - double(h));
+}
+
+// one pass of NV vectors of the double-float product (m of them stored)
+template <int NV>
+void launch_df(const Hamiltonian& h, const double* x, int ldx, double* y, int ldy, int m, float* stage,
+               cudaStream_t s) {
+  k_stage_df<NV><<<unsigned((h.n * NV + 255) / 256), 256, 0, s>>>(h.n, x, ldx, m, stage);
+  CG_CUDA(cudaGetLastError());
+  count_launch();
+  int nsm = 0;
+  CG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h.device));
+  constexpr int W = 8;
+  int per_sm = 0;
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm_df<NV, W>, W * 32, 0));
+  uint64_t ctas = uint64_t(nsm) * std::max(per_sm, 1);
+  uint64_t rpc = (h.n + ctas - 1) / ctas;
+  rpc = (rpc + W - 1) / W * W;
+  if (rpc == 0) rpc = W;
+  unsigned grid = unsigned((h.n + rpc - 1) / rpc);
+  if (grid)
+    k_spmm_df<NV, W><<<grid, W * 32, 0, s>>>(h.n, h.rowptr.p, h.col.p, h.hi.p, h.lo.p, stage, y, ldy, m, rpc);
+  CG_CUDA(cudaGetLastError());
+  count_launch();
 }
 
 // Launch shape of the FP32 product: WARPS warps per CTA, CTAS CTAs per SM,
@@ -474,37 +510,48 @@ __global__ void k_rm_to_cm(uint64_t n, int m, const T* __restrict__ src, int ld,
   dst[uint64_t(k) * n + i] = double(src[i * ld + k]);
 }
 
+// Device buffers of a host product: the column-major block, the packed operands
+// and, for REFINE, the staging rows.  They stay with the handle up to
+// kHostWorkKeep (allocating and freeing them took 0.6 of the 0.67 ms of a
+// 4-vector REFINE call on sd 5+6); larger ones are given back after the call.
+constexpr size_t kHostWorkKeep = size_t(256) << 20;
+
 template <class T>
 void spmm_host_t(const Hamiltonian& h, int precision, const double* x, double* y, int m) {
   const uint64_t n = h.n;
   cudaStream_t s = h.stream;
-  DBuf<double> cm(n * m);
-  cm.upload(x, n * m, s);
+  const int ldmax = (std::min(m, 16) + 3) / 4 * 4;
+  auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t bcm = up(n * m * sizeof(double)), bx = up(n * ldmax * sizeof(T));
+  const size_t bst = precision == CG_PREC_REFINE ? up(n * 16 * sizeof(float)) : 0;
+  DBuf<unsigned char>& ws = h.host_work;
+  if (ws.n < bcm + 2 * bx + bst) ws.alloc(bcm + 2 * bx + bst);
+  double* cm = reinterpret_cast<double*>(ws.p);
+  T* xi = reinterpret_cast<T*>(ws.p + bcm);
+  T* yi = reinterpret_cast<T*>(ws.p + bcm + bx);
+  CG_CUDA(cudaMemcpyAsync(cm, x, n * m * sizeof(double), cudaMemcpyHostToDevice, s));
   for (int c0 = 0; c0 < m; c0 += 16) {
     int mc = std::min(16, m - c0);
     int ld = (mc + 3) / 4 * 4;
-    DBuf<T> xi(n * ld), yi(n * ld);
     unsigned g = unsigned((n * mc + 255) / 256);
-    if (g) k_cm_to_rm<T><<<g, 256, 0, s>>>(n, mc, cm.p + uint64_t(c0) * n, xi.p, ld);
+    if (g) k_cm_to_rm<T><<<g, 256, 0, s>>>(n, mc, cm + uint64_t(c0) * n, xi, ld);
     CG_CUDA(cudaGetLastError());
     count_launch();
     if constexpr (std::is_same<T, double>::value) {
-      if (precision == CG_PREC_REFINE) {
-        DBuf<float> stage(n * 16);
-        spmm_refine_df(h, xi.p, ld, yi.p, ld, mc, stage.p, s);
-      } else {
-        spmm_launch(h, precision, xi.p, ld, yi.p, ld, mc, s);
-      }
+      if (precision == CG_PREC_REFINE)
+        spmm_refine_df(h, xi, ld, yi, ld, mc, reinterpret_cast<float*>(ws.p + bcm + 2 * bx), s);
+      else
+        spmm_launch(h, precision, xi, ld, yi, ld, mc, s);
     } else {
-      spmm_launch(h, precision, xi.p, ld, yi.p, ld, mc, s);
+      spmm_launch(h, precision, xi, ld, yi, ld, mc, s);
     }
-    if (g) k_rm_to_cm<T><<<g, 256, 0, s>>>(n, mc, yi.p, ld, cm.p + uint64_t(c0) * n);
+    if (g) k_rm_to_cm<T><<<g, 256, 0, s>>>(n, mc, yi, ld, cm + uint64_t(c0) * n);
     CG_CUDA(cudaGetLastError());
     count_launch();
-    CG_CUDA(cudaStreamSynchronize(s));
   }
-  CG_CUDA(cudaMemcpyAsync(y, cm.p, n * m * 8, cudaMemcpyDeviceToHost, s));
+  CG_CUDA(cudaMemcpyAsync(y, cm, n * m * 8, cudaMemcpyDeviceToHost, s));
   CG_CUDA(cudaStreamSynchronize(s));
+  if (ws.n > kHostWorkKeep) ws.release();
 }
 
 }  // namespace
@@ -680,23 +727,8 @@ void spmm_refine_df(const Hamiltonian& h, const double* x, int ldx, double* y, i
   if (h.precision != CG_PREC_FP32) throw Error(CG_ERR_ARG, "refinement product needs an FP32 (hi+lo) matrix");
   for (int c0 = 0; c0 < m; c0 += 8) {
     const int mc = std::min(8, m - c0);
-    k_stage_df<<<unsigned((h.n * 8 + 255) / 256), 256, 0, s>>>(h.n, x + c0, ldx, mc, stage);
-    CG_CUDA(cudaGetLastError());
-    count_launch();
-    int nsm = 0;
-    CG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h.device));
-    constexpr int W = 8;
-    int per_sm = 0;
-    CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm_df8<W>, W * 32, 0));
-    uint64_t ctas = uint64_t(nsm) * std::max(per_sm, 1);
-    uint64_t rpc = (h.n + ctas - 1) / ctas;
-    rpc = (rpc + W - 1) / W * W;
-    if (rpc == 0) rpc = W;
-    unsigned grid = unsigned((h.n + rpc - 1) / rpc);
-    if (grid)
-      k_spmm_df8<W><<<grid, W * 32, 0, s>>>(h.n, h.rowptr.p, h.col.p, h.hi.p, h.lo.p, stage, y + c0, ldy, mc, rpc);
-    CG_CUDA(cudaGetLastError());
-    count_launch();
+    if (mc <= 4) launch_df<4>(h, x + c0, ldx, y + c0, ldy, mc, stage, s);
+    else launch_df<8>(h, x + c0, ldx, y + c0, ldy, mc, stage, s);
   }
 }
 

@@ -592,8 +592,7 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
   if (ldx < m || ldy < m) throw Error(CG_ERR_ARG, "leading dimension smaller than the vector count");
   const uint64_t n = h.n;
   // n packed rows of 32 bytes in every precision, kept with the handle
-  DBuf<unsigned char>& pack = h.virt->pack;
-  if (n && !pack.p) pack.alloc(n * 32);
+  const DBuf<unsigned char>& pack = h.virt->pack;
   if (precision == CG_PREC_FP32) {
     float* w = reinterpret_cast<float*>(pack.p);
     const float* xf = static_cast<const float*>(x);
@@ -1146,6 +1145,7 @@ void virtual_build(const System& sys, const Operator& op, const Basis& b, int pr
   }
   CG_CUDA(cudaStreamSynchronize(s));
   v.err.alloc(1);
+  v.pack.alloc(b.n * 32);
   // FP32 products: the factored form where it is estimated faster than k_virtual
   // (40 us of launch and error read-back + 3.6 us per million elements for 8
   // vectors, within 20 % from sd 4 + 4 to fp 4 + 4).  8 vectors, factored /
