@@ -1159,13 +1159,14 @@ struct Engine {
     }
     t_abs += now() - t0;
   }
-  void diagonalize() {
+  // the projected problem: all Ritz values, and the `need` lowest vectors (default: the wanted ones)
+  void diagonalize(int need = 0) {
     double t0 = now();
     struct Acc { double& t; double t0; ~Acc() { t += now() - t0; } } acc_{t_eig, t0};
     std::vector<double> a(size_t(kpass) * kpass);
     for (int i = 0; i < kpass; ++i)
       for (int j = 0; j < kpass; ++j) a[size_t(i) * kpass + j] = S[size_t(i) * lim + j];
-    sym_eig(kpass, a, wall_, zvec);
+    sym_eig(kpass, a, wall_, zvec, std::max(need, nume));
     for (int i = 0; i < nume; ++i) eigs[i] = wall_[i];
   }
   double svec(int state, int row) const { return zvec[size_t(row) * kpass + state]; }
@@ -1485,7 +1486,7 @@ struct Engine {
     std::fill(eigs.begin(), eigs.end(), 0.0);
     for (;;) {
       for (int i = 0; i < nume; ++i) old[i] = eigs[i];
-      diagonalize();
+      diagonalize(kpass + mblock > lim ? keep : nume);
       if (kpass + mblock > lim) {
         double tc0 = now();
         int kp = std::min(keep, kpass);

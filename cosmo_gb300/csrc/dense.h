@@ -10,7 +10,9 @@ namespace cg {
 // the eigenvectors as columns: z[i*n + k] is component i of eigenvector k.
 // Householder tridiagonalisation followed by the implicit QL iteration, the
 // method of tav::EigenSystemT (include/tav/EigenSystem.cxx:49-69).
-void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::vector<double>& z);
+// need >= 0: only the need lowest eigenvectors are wanted; columns of z beyond
+// them may be zero.
+void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::vector<double>& z, int need = -1);
 
 // In-place Cholesky of the SPD n x n matrix a (row-major, lower factor in the
 // lower triangle).  Returns the index of the first non-positive pivot, or -1.
