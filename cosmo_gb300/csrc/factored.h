@@ -73,8 +73,8 @@ std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op
                                            cudaStream_t s);
 constexpr uint64_t kFactoredMaxWork = 32ull << 30;
 // stored matrices of fewer entries keep the row-wise product without an estimate
-// (their rows are read from L2; the largest sd sector has 2.5e7)
-constexpr uint64_t kFactoredMinEntries = 1ull << 25;
+// (fp 2+4, 3.3e7 entries: 120 us row-wise, 60 factored; sd 4+4, 6e6: 24 and 33)
+constexpr uint64_t kFactoredMinEntries = 1ull << 24;
 
 // Y = H X from x packed as n rows of 8 FP32 vectors (32-byte aligned).
 // Asynchronous; allocates nothing.
