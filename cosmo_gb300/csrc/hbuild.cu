@@ -26,6 +26,7 @@
 
 #include "device.h"
 #include "factored.h"
+#include "rowtab.h"
 #include "tiled.h"
 
 namespace cg {
@@ -455,6 +456,10 @@ __global__ void k_max_u32(const uint32_t* __restrict__ a, uint64_t n, unsigned* 
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
+// rows from which the sorted move tables (rowtab.h) are worth their set-up (whole
+// build: 4,000 rows of fp 2+2 1.29 ms either way, 6,116 of sd 3+3 1.05 -> 0.95)
+constexpr uint64_t kRowTableMin = 4096;
+
 }  // namespace
 
 void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, int precision, Hamiltonian& h,
@@ -475,6 +480,7 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
 
   DevOperator dop;
   std::unique_ptr<WideRows> wide;
+  std::unique_ptr<RowTables> tab;
   std::vector<int8_t> m2(b.ns);
   for (int i = 0; i < b.ns; ++i) m2[i] = int8_t(b.sp_m2[i]);
   DBuf<int8_t> dm2;
@@ -509,9 +515,13 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
   if (grid == 0) grid = 1;
   DBuf<int> derr(1);
   CG_CUDA(cudaMemsetAsync(derr.p, 0, sizeof(int), s));
+  if (!wide && n >= kRowTableMin) {
+    tab = row_tables(b, dop, s);
+    if (tab && !tab->count(counts.p)) tab.reset();
+  }
   if (wide) {
     wide->count(counts.p, derr.p);
-  } else {
+  } else if (!tab) {
     k_count<<<grid, T, 0, s>>>(c, b.binom.p, counts.p, derr.p);
     CG_CUDA(cudaGetLastError());
     count_launch();
@@ -551,11 +561,12 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
   counts.release();
 
   h.col.alloc(std::max<uint64_t>(h.nnz, 1));
-  DBuf<double> tmpval(std::max<uint64_t>(h.nnz, 1));
+  DBuf<double> tmpval;
+  if (!tab) tmpval.alloc(std::max<uint64_t>(h.nnz, 1));
   h.diag.alloc(std::max<uint64_t>(n, 1));
   if (n && wide) {
     wide->fill(h.rowptr.p, h.col.p, tmpval.p, h.diag.p);
-  } else if (n) {
+  } else if (n && !tab) {
     k_fill<<<grid, T, 0, s>>>(c, b.binom.p, h.rowptr.p, h.col.p, tmpval.p, h.diag.p);
     CG_CUDA(cudaGetLastError());
     count_launch();
@@ -567,14 +578,16 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
     h.lo.alloc(std::max<uint64_t>(h.nnz, 1));
   }
   int L = 1;
-  while (L < h.max_row) L <<= 1;
+  while (!tab && L < h.max_row) L <<= 1;
   size_t smem = size_t(L) * 16;
   if (smem > 200 * 1024) throw Error(CG_ERR_UNSUPPORTED, "row longer than the per-row sort supports");
   if (smem > 48 * 1024)
     CG_CUDA(cudaFuncSetAttribute(k_sort_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   DBuf<unsigned long long> dup(1);
   CG_CUDA(cudaMemsetAsync(dup.p, 0, 8, s));
-  if (n) {
+  if (tab) {
+    tab->fill(h.rowptr.p, h.col.p, h.val64.p, h.hi.p, h.lo.p, h.diag.p, dup.p);
+  } else if (n) {
     // rows of up to 1024 entries: warp-per-row register sort; longer rows
     // (or 2^22 rows and more, whose columns need more than 22 key bits):
     // CTA-per-row shared-memory sort
@@ -608,11 +621,14 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
   h.blocks.push_back(b.n);
   if (precision == CG_PREC_FP32 && tiled_copy && h.nnz >= kFactoredMinEntries) {
     // Products of up to 8 vectors: the factored form where it is estimated
-    // faster than the stored values (5 us + 3.2 us per million entries row-wise,
-    // 1.9 us block-tiled: fp 4+4 2.42 ms tiled, 1.42 factored; fp 3+4 0.54 and
-    // 0.29; fp 3+3 0.16 row-wise, 0.07)
+    // faster than the stored values: 3.4 us per million entries row-wise, 1.9 us
+    // block-tiled with long blocks and more with short ones (fp 4+4, 405 rows a
+    // block: 2.42 ms tiled, 1.42 factored; fp 4+3, 100 rows: 0.59 and 0.27; fp 5+2,
+    // 17 rows: 0.54, row-wise 0.41 and 0.23; fp 3+3: row-wise 0.16 and 0.07)
     const auto t0 = std::chrono::steady_clock::now();
-    h.fact = factored_build(sys, op, b, 5 + (h.nnz >= kTiledMinEntries ? 1.9e-6 : 3.2e-6) * double(h.nnz), s);
+    const double per_block = double(n) / double(std::max<size_t>(b.h_bstart.size(), 1));
+    const double per_entry = h.nnz >= kTiledMinEntries ? std::min(3.4e-6, 1.9e-6 * (1 + 40 / per_block)) : 3.4e-6;
+    h.fact = factored_build(sys, op, b, 5 + per_entry * double(h.nnz), s);
     if (h.fact) h.format = CG_FORMAT_FACTORED;
     h.build_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
