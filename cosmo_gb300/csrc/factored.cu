@@ -66,14 +66,14 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // FP32 product of 8 vectors, neutron + proton pairs.  Bound by the FP32 pipe in
 // principle (fp 4 + 4: 1.7e9 multiply-adds x 8 with filled-up tiles, 0.35 ms); it
-// takes 0.89 ms, the pipe 48 % busy, the rest waiting at the two barriers of a
-// chunk.  Four warps a CTA and four CTAs an SM measured best (3, 5, 6, 8 warps:
-// 1.00, 0.91, 0.98, 1.10 ms; rows fetched in two alternating halves 0.90).
-// A warp forms tiles of 2 groups of OT outputs (8, or 4 for a remainder of at
-// most 8) x 16 spectators.  The lane's bit 1 picks the group and the other bits
-// the spectator: lanes i and i ^ 1 read the same piece of the matrix and lanes
-// i and i ^ 2 the same piece of x, so that every 16-byte shared-memory read of
-// the warp takes two cycles instead of four.
+// takes 0.84 ms, the rest waiting at the two barriers of a chunk.  Four warps a
+// CTA and four CTAs an SM measured best (3, 5, 6, 8 warps with tiles of 8: 1.00,
+// 0.91, 0.98, 1.10 ms against 0.89; rows fetched in two alternating halves 0.90).
+// A warp forms tiles of 2 groups of OT <= 8 outputs x 16 spectators (fact_tiles).
+// The lane's bit 1 picks the group and the other bits the spectator: lanes i and
+// i ^ 1 read the same piece of the matrix and lanes i and i ^ 2 the same piece of
+// x, so that every 16-byte shared-memory read of the warp takes two cycles
+// instead of four.
 constexpr int kFW = 4;  // warps
 
 // shared-memory head of the FP32 kernels: the pairs of the job
@@ -83,50 +83,46 @@ struct alignas(16) FHead32 {
   uint32_t meta[kFMaxPairs];
 };
 
-// acc += matrix rows [0, kn) x gathered rows; sp holds the spectator's phase of
-// each (pair, spectator) as a sign bit, applied to the matrix values while
-// they are doubled for the packed multiply-adds
+// One warp tile: acc += matrix rows x gathered rows, then the output rows.  sg
+// holds the spectator's phase of each (pair, spectator) as a sign bit, applied
+// to the matrix values while they are doubled for the packed multiply-adds.
+// A group's OT values lie in 8 places, so that two 16-byte reads fetch them.
 template <int OT>
-__device__ __forceinline__ void mac32(float2 (&acc)[OT][4], const float* wp, int wld, const float4* xp,
-                                      const uint32_t* sp, int ld, int kn) {
-#pragma unroll 2
-  for (int k = 0; k < kn; ++k) {
-    const float4 x0 = xp[0], x1 = xp[ld];
-    const uint32_t f = *sp;
-    const float2 xv[4] = {{x0.x, x0.y}, {x0.z, x0.w}, {x1.x, x1.y}, {x1.z, x1.w}};
-#pragma unroll
-    for (int q = 0; q < OT / 4; ++q) {
-      const float4 t = reinterpret_cast<const float4*>(wp)[q];
-      const float wv[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float w1 = __uint_as_float(__float_as_uint(wv[u]) ^ f);
-        const float2 w2 = make_float2(w1, w1);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) fma2(acc[4 * q + u][v], w2, xv[v]);
-      }
-    }
-    wp += wld;
-    xp += 2 * ld;
-    sp += ld;
-  }
-}
-
-template <int OT>
-__device__ __forceinline__ void tile32(const FArgs& a, const FHead32& hd, int D, int o0, int j, bool live,
+__device__ __forceinline__ void tile32(const FArgs& a, const FHead32& hd, int D, int tile, int j, bool live,
                                        const float* ws, int wld, const float4* xs, const uint32_t* sg, int ld,
                                        const uint32_t* of, unsigned char* __restrict__ z) {
-  const int og = o0 + ((threadIdx.x >> 1) & 1) * OT;
+  const int group = tile * 2 + ((threadIdx.x >> 1) & 1);
   float2 acc[OT][4];
 #pragma unroll
   for (int t = 0; t < OT; ++t)
 #pragma unroll
     for (int v = 0; v < 4; ++v) acc[t][v] = make_float2(0.f, 0.f);
-  mac32<OT>(acc, ws + og, wld, xs + j, sg + j, ld, D);
+  const float* wp = ws + group * 8;
+  const float4* xp = xs + j;
+  const uint32_t* sp = sg + j;
+#pragma unroll 2
+  for (int k = 0; k < D; ++k) {
+    const float4 x0 = xp[0], x1 = xp[ld];
+    const uint32_t f = *sp;
+    const float2 xv[4] = {{x0.x, x0.y}, {x0.z, x0.w}, {x1.x, x1.y}, {x1.z, x1.w}};
+    const float4 w0 = reinterpret_cast<const float4*>(wp)[0];
+    const float4 w1 = OT > 4 ? reinterpret_cast<const float4*>(wp)[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+    for (int t = 0; t < OT; ++t) {
+      const float ws1 = __uint_as_float(__float_as_uint(wv[t]) ^ f);
+      const float2 w2 = make_float2(ws1, ws1);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) fma2(acc[t][v], w2, xv[v]);
+    }
+    wp += wld;
+    xp += 2 * ld;
+    sp += ld;
+  }
   if (!live) return;
 #pragma unroll
   for (int t = 0; t < OT; ++t) {
-    const int k = og + t;
+    const int k = group * OT + t;
     if (k < D) {
       const uint32_t o = of[hd.src[k].y];
       if (o != ~0u) {
@@ -144,6 +140,11 @@ __device__ __forceinline__ void tile32(const FArgs& a, const FHead32& hd, int D,
   }
 }
 
+// Outputs of a job in 1, 2 or 4 warp tiles (more above 64 pairs) of 2 groups of
+// OT, as even as they can be: with tiles of 16 one of the four warps was idle
+// for 33 to 48 pairs, half of the work of fp 4 + 4 (0.89 ms; now 0.84).
+__host__ __device__ inline int fact_tiles(int D) { return D <= 16 ? 1 : D <= 32 ? 2 : D <= 64 ? 4 : (D + 15) / 16; }
+
 __global__ void __launch_bounds__(kFW * 32, 4) k_fact32(FArgs a, const float* __restrict__ w,
                                                         const unsigned char* __restrict__ x,
                                                         unsigned char* __restrict__ z, int smem) {
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(kFW * 32, 4) k_fact32(FArgs a, const float* __
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const FJob job = a.jobs[blockIdx.x];
   const int count = int(job.count), cols = a.cols, D = int(job.npair);
-  const int ot = (D + 15) >> 4, wld = ((D + 7) >> 3) * 8;
+  const int ot = fact_tiles(D), OT = (D + 2 * ot - 1) / (2 * ot), wld = ot * 16;
   // spectators of a chunk: as many groups of 16 as fill the warps, within the shared memory
   const int cap = (smem - int(sizeof(FHead32)) - D * wld * 4) / (D * 36 + 2 * cols * 4) >> 4;
   const int NK = min(min(max(kFW / ot, 1), cap), (count + 15) >> 4) * 16;
@@ -171,14 +172,16 @@ __global__ void __launch_bounds__(kFW * 32, 4) k_fact32(FArgs a, const float* __
   }
   __syncthreads();
   // the matrix restricted to the job's pairs, phases of both sides folded in; a warp per row
-  for (int o = lane; o < wld; o += 32) {
-    const uint32_t mo = o < D ? hd.meta[o] : 0;
+  for (int i = lane; i < wld; i += 32) {
+    const int o = (i >> 3) * OT + (i & 7);
+    const bool used = (i & 7) < OT && o < D;
+    const uint32_t mo = used ? hd.meta[o] : 0;
     const float* src = w + job.w0 + meta_idx(mo);
 #pragma unroll 8
     for (int k = warp; k < D; k += kFW) {
       const uint32_t mk = hd.meta[k];
-      const float v = o < D ? __ldg(src + meta_idx(mk) * job.ldw) : 0.f;
-      ws[k * wld + o] = __uint_as_float(__float_as_uint(v) ^ ((mk ^ mo) & 0x80000000u));
+      const float v = used ? __ldg(src + meta_idx(mk) * job.ldw) : 0.f;
+      ws[k * wld + i] = __uint_as_float(__float_as_uint(v) ^ ((mk ^ mo) & 0x80000000u));
     }
   }
   cp_async_wait_all();
@@ -209,15 +212,21 @@ __global__ void __launch_bounds__(kFW * 32, 4) k_fact32(FArgs a, const float* __
     for (int i = tid; i < left; i += NT) cp_async4(nxt + i, stab + i);
     cp_async_wait_all();
     __syncthreads();
-    for (int jt = 0, o0 = warp * 16; jt * 16 < cnt; o0 += kFW * 16) {
-      while (o0 >= ot * 16) {
-        o0 -= ot * 16;
-        ++jt;
+    const int tiles = ot * ((cnt + 15) >> 4);
+    for (int t = warp; t < tiles; t += kFW) {
+      const int jt = t / ot, j = jt * 16 + jl, tile = t - jt * ot;
+#define CG_TILE(N) tile32<N>(a, hd, D, tile, j, j < cnt, ws, wld, xs, sg, NK, cur + j * cols, z)
+      switch (OT) {
+        case 8: CG_TILE(8); break;
+        case 7: CG_TILE(7); break;
+        case 6: CG_TILE(6); break;
+        case 5: CG_TILE(5); break;
+        case 4: CG_TILE(4); break;
+        case 3: CG_TILE(3); break;
+        case 2: CG_TILE(2); break;
+        default: CG_TILE(1); break;
       }
-      const int j = jt * 16 + jl;
-      if (jt * 16 >= cnt) break;
-      if (D - o0 > 8) tile32<8>(a, hd, D, o0, j, j < cnt, ws, wld, xs, sg, NK, cur + j * cols, z);
-      else tile32<4>(a, hd, D, o0, j, j < cnt, ws, wld, xs, sg, NK, cur + j * cols, z);
+#undef CG_TILE
     }
     uint32_t* t = cur;
     cur = nxt;
@@ -543,7 +552,7 @@ std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op
   if (f.dmax > kFMaxPairs || f.dmax_same > kFPairs || w.size() >= (1ull << 31) || list.size() >= (1ull << 32))
     return nullptr;
   // at least 16 spectators a chunk beside the largest matrix
-  f.smem32 = std::max(kFSmem, int(sizeof(FHead32)) + f.dmax * ((f.dmax + 7) / 8) * 32 +
+  f.smem32 = std::max(kFSmem, int(sizeof(FHead32)) + f.dmax * fact_tiles(f.dmax) * 64 +
                                   16 * (f.dmax * 36 + 2 * f.cols * 4));
   if (f.smem32 > 227 * 1024) return nullptr;
   // few jobs: split their spectators (whole tiles of 16, or 64 rows) until there are some per CTA slot
@@ -579,7 +588,7 @@ std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op
   }
   f.njobs = jobs.size();
   // Time of one product in us, fitted to sd and fp systems of 28 to 1,963,461
-  // rows (fp 4 + 4: 0.89 + 0.26 + 0.26 ms; sd 6 + 6: 98 + 46 + 27 us): the
+  // rows (fp 4 + 4: 0.84 + 0.26 + 0.26 ms; sd 6 + 6: 98 + 46 + 27 us): the
   // multiply-adds and the start of each job, and the partial sums read back.
   f.est_us = 12 + 4.7e-7 * f.macs + 6.5e-3 * f.njobs_pn + 3e-7 * f.macs_same + 7e-3 * (f.njobs - f.njobs_pn) +
              double(slots) * b.n * 32 / 6.5e6;

@@ -1149,7 +1149,7 @@ void virtual_build(const System& sys, const Operator& op, const Basis& b, int pr
   // FP32 products: the factored form where it is estimated faster than k_virtual
   // (40 us of launch and error read-back + 3.6 us per million elements for 8
   // vectors, within 20 % from sd 4 + 4 to fp 4 + 4).  8 vectors, factored /
-  // k_virtual: fp 4 + 4 1.40 / 4.34 ms, fp 5 + 3 1.02 / 3.75, fp 3 + 3 0.07 / 0.26,
+  // k_virtual: fp 4 + 4 1.36 / 4.34 ms, fp 5 + 3 1.02 / 3.75, fp 3 + 3 0.07 / 0.26,
   // sd 3 + 3 15 / 49 us; near half filling most pairs of a core are blocked and
   // k_virtual stays (sd 6 + 6 172 / 129 us, sd 8 + 8 149 / 67).
   h.fact = factored_build(sys, op, b, 40 + 3.6e-6 * double(conn), s);
