@@ -26,6 +26,8 @@
 #include <numeric>
 #include <type_traits>
 
+#include <cooperative_groups.h>
+
 #include "batched.h"
 #include "dfloat.h"
 #include "dense.h"
@@ -67,9 +69,9 @@ __global__ void k_dense_fill(int n, uint64_t r0, const uint64_t* __restrict__ rp
 // computed in R: FP64 (off-diagonal norm down to 1e-12 of the Frobenius norm)
 // or FP32 (1e-6).  FP32 vectors alone, off by ~eps32 |S| / gap, kept the
 // FP32 Davidson phase from reaching its 1e-4 residuals (300 instead of 133
-// iterations), so that phase runs the FP32 Jacobi and then the FP64 one from
-// its vectors (re-orthonormalized: ortho), which leaves the FP64 pipe only
-// one or two sweeps.  Cyclic Jacobi with the round-robin ordering: each round
+// iterations), so that phase runs the FP32 Jacobi and refines its vectors to
+// FP64 (k_brefine); the FP64 Jacobi takes the matrices where that fails, from
+// the FP32 vectors (re-orthonormalized: ortho).  Cyclic Jacobi with the round-robin ordering: each round
 // applies k/2 disjoint rotations at once, skipping those whose |a_pq| is
 // below 1e-17 (FP32: 1e-7) of sqrt|a_pp a_qq|; at most 40 sweeps.
 template <class R>
@@ -86,11 +88,13 @@ constexpr size_t jac_smem() {
 template <class R>
 __global__ void __launch_bounds__(256) k_bjacobi(const double* __restrict__ Ain, const int* __restrict__ kdim,
                                                  int kconst, double* __restrict__ w, double* Zout,
-                                                 const int* __restrict__ fz, int kprev, int ortho) {
+                                                 const int* __restrict__ fz, int kprev, int ortho,
+                                                 const int* __restrict__ solved) {
   constexpr R kConv = sizeof(R) == 4 ? R(1e-12) : R(1e-24);   // (off / total)^2 at convergence
   constexpr R kTiny = sizeof(R) == 4 ? R(1e-30) : R(1e-300);
   constexpr R kSkip = sizeof(R) == 4 ? R(1e-7) : R(1e-17);
   if (fz && fz[blockIdx.x]) return;
+  if (solved && solved[blockIdx.x]) return;  // by k_brefine
   extern __shared__ __align__(16) unsigned char jsm_raw[];
   R* jsm = reinterpret_cast<R*>(jsm_raw);
   R(*A)[kJac + 1] = reinterpret_cast<R(*)[kJac + 1]>(jsm);
@@ -279,6 +283,129 @@ __global__ void __launch_bounds__(256) k_bjacobi(const double* __restrict__ Ain,
   for (int i = tid; i < kJac * kJac; i += blockDim.x) {
     const int r = i / kJac, c = i % kJac;
     Zb[r * kJac + c] = (r < k && c < k) ? double(Z[r][order[c]]) : 0.0;
+  }
+}
+
+// ------------------------------------------- refinement of FP32 eigenvectors
+// FP64 eigenvectors of a k x k matrix from the FP32 ones in Zout: with
+// R = I - Z^T Z, S = Z^T A Z and lam_j = S_jj / (1 - R_jj), the columns of
+// Z + Z E, E_ij = (S_ij + lam_j R_ij) / (lam_j - lam_i), E_jj = R_jj / 2, have
+// the square of the former error (Ogita & Aishima, Japan J. Indust. Appl.
+// Math. 35, 2018).  Repeated until ||E||_F <= 1e-8, so that what is left is
+// below FP64 rounding; a pair whose coupling is rounding error keeps
+// E_ij = R_ij / 2.  Where close eigenvalues keep E from shrinking, solved = 0
+// and the FP32 vectors stay: the Jacobi sweeps take those.
+//
+// Bound by the FP64 pipe (2 multiply-adds per clock and SM): 5 k^3 a pass,
+// where a Jacobi sweep has about 6 k^3 and k serial rounds of square roots.  A
+// cluster holds A and Z in every CTA and splits the columns, so that only the
+// updated columns are exchanged (distributed shared memory).  24 problems, k up
+// to 40, clusters of 6: 45 us on average, where the FP64 sweeps from the FP32
+// vectors took 416.
+constexpr int kRefinePasses = 5;
+constexpr int kRefineCtas = 8;  // largest cluster
+constexpr int kRefineLd = kMaxLim + 1;
+constexpr size_t kRefineSmem = (size_t(5) * kMaxLim * kRefineLd + kMaxLim + kRefineCtas + 8) * sizeof(double);
+
+__global__ void __launch_bounds__(256) k_brefine(const double* __restrict__ Ain, int k, double* __restrict__ w,
+                                                 double* Zout, const int* __restrict__ fz,
+                                                 int* __restrict__ solved) {
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int C = int(cl.num_blocks()), me = int(cl.block_rank());
+  const int p = int(blockIdx.x) / C, tid = threadIdx.x;
+  if (fz[p]) return;  // the whole cluster
+  extern __shared__ __align__(16) unsigned char rsm_raw[];
+  double(*A)[kRefineLd] = reinterpret_cast<double(*)[kRefineLd]>(rsm_raw);
+  double(*Z)[kRefineLd] = A + kMaxLim;
+  double(*Y)[kRefineLd] = Z + kMaxLim;  // own columns, column c0 + c in row c: A Z, then the update
+  double(*E)[kRefineLd] = Y + kMaxLim;  // S, then E
+  double(*G)[kRefineLd] = E + kMaxLim;  // R
+  double* lam = &G[kMaxLim][0];
+  double* esum = lam + kMaxLim;      // ||E||^2 of every CTA's columns
+  double* red = esum + kRefineCtas;  // of every warp
+  const auto block_sum = [&](double v) {
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((tid & 31) == 0) red[tid >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int i = 0; i < 8; ++i) t += red[i];
+    return t;
+  };
+  const double* Ab = Ain + size_t(p) * kJac * kJac;
+  double* Zb = Zout + size_t(p) * kJac * kJac;
+  double fro = 0.0;
+  for (int i = tid; i < k * k; i += 256) {
+    const int r = i / k, c = i - r * k;
+    const double v = Ab[r * kJac + c];
+    A[r][c] = v;
+    Z[r][c] = Zb[r * kJac + c];
+    fro += v * v;
+  }
+  const double tiny = 2e-16 * sqrt(block_sum(fro));
+  const int c0 = me * k / C, nc = (me + 1) * k / C - c0;
+  bool ok = false;
+  cl.sync();  // every CTA of the cluster runs and has read Zout
+  for (int pass = 0; pass < kRefinePasses && !ok; ++pass) {
+    for (int i = tid; i < k * nc; i += 256) {
+      const int c = i / k, r = i - c * k;
+      double v = 0.0;
+      for (int t = 0; t < k; ++t) v += A[r][t] * Z[t][c0 + c];
+      Y[c][r] = v;
+    }
+    __syncthreads();
+    for (int i = tid; i < k * nc; i += 256) {
+      const int c = i / k, r = i - c * k;
+      double sv = 0.0, g = 0.0;
+      for (int t = 0; t < k; ++t) {
+        sv += Z[t][r] * Y[c][t];
+        g += Z[t][r] * Z[t][c0 + c];
+      }
+      E[c][r] = sv;
+      G[c][r] = (r == c0 + c ? 1.0 : 0.0) - g;
+      if (r == c0 + c) {
+        const double l = sv / g;
+        for (int b = 0; b < C; ++b) cl.map_shared_rank(lam, b)[r] = l;
+      }
+    }
+    cl.sync();  // lam
+    double e2 = 0.0;
+    for (int i = tid; i < k * nc; i += 256) {
+      const int c = i / k, r = i - c * k;
+      const double num = E[c][r] + lam[c0 + c] * G[c][r];
+      const double e = (r == c0 + c || fabs(num) <= tiny) ? 0.5 * G[c][r] : num / (lam[c0 + c] - lam[r]);
+      E[c][r] = e;
+      e2 += e * e;
+    }
+    e2 = block_sum(e2);
+    if (tid < C) cl.map_shared_rank(esum, tid)[me] = e2;
+    for (int i = tid; i < k * nc; i += 256) {
+      const int c = i / k, r = i - c * k;
+      double v = 0.0;
+      for (int t = 0; t < k; ++t) v += Z[r][t] * E[c][t];
+      Y[c][r] = Z[r][c0 + c] + v;
+    }
+    cl.sync();  // esum, and nobody reads Z any more
+    double tot = 0.0;
+    for (int b = 0; b < C; ++b) tot += esum[b];
+    if (!(tot < 0.01)) break;  // the same in every CTA; also for NaN
+    ok = tot <= 1e-16;
+    for (int i = tid; i < k * nc; i += 256) {
+      const int c = i / k, r = i - c * k;
+      for (int b = 0; b < C; ++b) cl.map_shared_rank(&Z[r][c0 + c], b)[0] = Y[c][r];
+    }
+    cl.sync();  // Z
+  }
+  if (me == 0 && tid == 0) solved[p] = ok;
+  if (!ok) return;
+  // ascending order (ties by index)
+  for (int c = tid >> 5; c < nc; c += 8) {
+    const double l = lam[c0 + c];
+    int rank = 0;
+    for (int j = tid & 31; j < k; j += 32) rank += lam[j] < l || (lam[j] == l && j < c0 + c);
+    rank = __reduce_add_sync(0xffffffffu, rank);
+    if ((tid & 31) == 0) w[size_t(p) * kJac + rank] = l;
+    for (int r = tid & 31; r < k; r += 32) Zb[r * kJac + rank] = Z[r][c0 + c];
   }
 }
 
@@ -742,12 +869,12 @@ template <class T>
 struct BEngine {
   BatchSet& bs;
   cudaStream_t s;
-  int Q, nev, b, lim, keep;
+  int Q, nev, b, lim, keep, nsm = 0;
   uint32_t N;
   DBuf<T> V, AV, R, W;        // N x lim, N x lim, N x 8, N x 8 (SpMM staging, FP32 engine)
   DBuf<double> S, Z, w, G, M, part, rnorm;
   DBuf<float> dfstage;        // N x 16 (FP64 engine: double-float staging)
-  DBuf<int> fz, kfreeze, nconv, bad;
+  DBuf<int> fz, kfreeze, nconv, bad, solved;
   int* h_nconv = nullptr;     // pinned
   std::vector<cudaGraphExec_t> graphs;  // per basis size
   std::vector<int> graph_kernels;
@@ -758,6 +885,7 @@ struct BEngine {
 
   BEngine(BatchSet& b_, int nev0, int b0, int lim0, int keep0)
       : bs(b_), s(b_.stream), Q(b_.nq), nev(nev0), b(b0), lim(lim0), keep(keep0), N(uint32_t(b_.H.n)) {
+    CG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, bs.device));
     V.alloc(size_t(N) * lim);
     AV.alloc(size_t(N) * lim);
     R.alloc(size_t(N) * 8);
@@ -774,6 +902,7 @@ struct BEngine {
     kfreeze.alloc(Q);
     nconv.alloc(1);
     bad.alloc(Q);
+    solved.alloc(Q);
     CG_CUDA(cudaMallocHost(&h_nconv, sizeof(int)));
     CG_CUDA(cudaMemsetAsync(V.p, 0, V.bytes(), s));
     CG_CUDA(cudaMemsetAsync(AV.p, 0, AV.bytes(), s));
@@ -823,6 +952,22 @@ struct BEngine {
       k_bfill<T><<<nblk(N), 256, 0, s>>>(N, bs.rowprob.p, bad.p, V.p, lim, c0, b, 0x1234567u + pass, fz.p);
     }
   }
+  // FP64 eigenvectors from the FP32 ones in Z; as many CTAs a problem as the
+  // batch leaves SMs for
+  void refine(int k) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {unsigned(std::clamp(nsm / Q, 1, kRefineCtas)), 1, 1};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(Q) * at.val.clusterDim.x);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = kRefineSmem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CG_CUDA(cudaLaunchKernelEx(&cfg, k_brefine, static_cast<const double*>(S.p), k, w.p, Z.p,
+                               static_cast<const int*>(fz.p), solved.p));
+  }
   // one iteration with current basis size k (the newest b columns not yet multiplied)
   void enqueue_step(int k, double tol) {
     spmm(k - b);
@@ -830,14 +975,14 @@ struct BEngine {
     k_bset_proj<<<Q, 128, 0, s>>>(k, b, k - b, G.p, S.p, fz.p);
     // warm start from the previous step's eigenvectors (size k - b; after a
     // restart the kept block is diagonal and Z's leading block the identity).
-    // FP32 phase: FP32 sweeps first, then FP64 sweeps from their
-    // (re-orthonormalized) vectors, which leave only ~1e-7 couplings, so the
-    // FP64 pipe does one or two sweeps instead of a full solve
+    // FP32 phase: FP32 sweeps, their vectors refined to FP64; FP64 sweeps only
+    // where the refinement did not converge
     if (sizeof(T) == 4) {
-      k_bjacobi<float><<<Q, 256, jac_smem<float>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0);
-      k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k, 1);
+      k_bjacobi<float><<<Q, 256, jac_smem<float>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0, nullptr);
+      refine(k);
+      k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k, 1, solved.p);
     } else {
-      k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0);
+      k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0, nullptr);
     }
     k_bresid<T><<<unsigned(bs.nchunks), 256, 0, s>>>(bs.chunks.p, V.p, AV.p, lim, k, w.p, Z.p, R.p, 8, b, fz.p);
     xty(R.p, 8, 0, b, R.p, 8, 0, b);
@@ -1030,6 +1175,7 @@ void batch_solve(BatchSet& bs, const BatchParams& prm, BatchResult& res) {
   // (also loads both Jacobi kernels before any iteration is captured into a graph)
   CG_CUDA(cudaFuncSetAttribute(k_bjacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(jac_smem<double>())));
+  CG_CUDA(cudaFuncSetAttribute(k_brefine, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRefineSmem)));
   CG_CUDA(cudaFuncSetAttribute(k_bjacobi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(jac_smem<float>())));
   if (prm.nev < 1 || prm.nev > kMaxB) throw Error(CG_ERR_ARG, "batched solve: nstates must be in 1..8");
@@ -1050,7 +1196,7 @@ void batch_solve(BatchSet& bs, const BatchParams& prm, BatchResult& res) {
     DBuf<double> w(size_t(bs.nd) * kJac), Z(size_t(bs.nd) * kJac * kJac);
     DBuf<int> kd;
     kd.upload(bs.ddim, s);
-    k_bjacobi<double><<<bs.nd, 256, jac_smem<double>(), s>>>(bs.dense.p, kd.p, 0, w.p, Z.p, nullptr, 0, 0);
+    k_bjacobi<double><<<bs.nd, 256, jac_smem<double>(), s>>>(bs.dense.p, kd.p, 0, w.p, Z.p, nullptr, 0, 0, nullptr);
     CG_CUDA(cudaGetLastError());
     count_launch();
     dw.resize(size_t(bs.nd) * kJac);
