@@ -721,15 +721,16 @@ __global__ void __launch_bounds__(64) k_bpip(int Q, int c0, int b, const double*
                                               double* __restrict__ M, int* __restrict__ bad,
                                               const int* __restrict__ fz, double min_ratio) {
   // one CTA of 64 threads per problem: the b x b Gram correction and the
-  // (c0 + b) x b coefficients in parallel, the b x b factorisation on thread 0
+  // (c0 + b) x b coefficients by all, the factorisation by one lane per row and
+  // the triangular solves by one lane per column.  Bound by the latency of FP64
+  // square roots and divisions (80 us when one thread did them all; 24 us).
   const int q = blockIdx.x, tid = threadIdx.x;
   if (q >= Q) return;
   if (fz[q]) {
     if (tid == 0) bad[q] = 0;
     return;
   }
-  __shared__ double w[kMaxLim * kMaxB], S[kMaxB][kMaxB], R[kMaxB][kMaxB], d[kMaxB];
-  __shared__ int bmask;
+  __shared__ double w[kMaxLim * kMaxB], S[kMaxB][kMaxB], R[kMaxB][kMaxB], L[kMaxB][kMaxB], d[kMaxB];
   const int K = c0 + b;
   for (int i = tid; i < K * b; i += blockDim.x) w[i] = G[size_t(q) * (kMaxLim * kMaxB) + i];
   __syncthreads();
@@ -745,59 +746,48 @@ __global__ void __launch_bounds__(64) k_bpip(int Q, int c0, int b, const double*
     S[i][j] = v * d[i] * d[j];
   }
   __syncthreads();
-  if (tid == 0) {
-    int weak = 0, badmask = 0;
+  if (tid < 32) {  // row (then column) tid of the b x b matrices
+    const unsigned all = 0xffffffffu;
+    const bool row = tid < b;
+    const bool zero = row && !(d[tid] > 0.0);
+    const bool small = row && !zero && !(S[tid][tid] >= min_ratio);
+    // nothing outside the basis
+    const int badmask = int(__ballot_sync(all, zero || (small && !(S[tid][tid] > 1e-24))));
+    int proj = int(__ballot_sync(all, small)) | badmask;  // columns that are only projected
+    const int skip = proj;
+    // Cholesky of S on the healthy columns (the others: identity)
     for (int j = 0; j < b; ++j) {
-      if (!(d[j] > 0.0)) badmask |= 1 << j;
-      else if (!(S[j][j] >= min_ratio)) {
-        weak |= 1 << j;
-        if (!(S[j][j] > 1e-24)) badmask |= 1 << j;  // nothing outside the basis
-      }
+      const bool live = row && tid >= j && !(skip >> tid & 1) && !(skip >> j & 1);
+      double sum = live ? S[tid][j] : 0.0;
+      if (live)
+        for (int t = 0; t < j; ++t) sum -= L[tid][t] * L[j][t];
+      // numerically dependent on the columns before: project only
+      if (__ballot_sync(all, tid == j && live && !(sum > 1e-24))) proj |= 1 << j;
+      if (tid == j) L[j][j] = proj >> j & 1 ? 1.0 : sqrt(sum);
+      __syncwarp();
+      if (row && tid > j) L[tid][j] = live && !(proj >> j & 1) ? sum / L[j][j] : 0.0;
+      if (tid == j && (proj >> j & 1))
+        for (int t = 0; t < j; ++t) L[j][t] = 0.0;
+      __syncwarp();
     }
-    const int skip = weak | badmask;
-    // Cholesky of S on the healthy columns (skipped rows/columns: identity)
-    double L[kMaxB][kMaxB];
-    for (int i = 0; i < b; ++i)
-      for (int j = 0; j <= i; ++j) {
-        if ((skip >> i & 1) || (skip >> j & 1)) {
-          L[i][j] = i == j ? 1.0 : 0.0;
-          continue;
-        }
-        double sum = S[i][j];
-        for (int t = 0; t < j; ++t) sum -= L[i][t] * L[j][t];
-        if (i == j) {
-          if (!(sum > 1e-24)) {  // numerically dependent on the columns before: project only
-            weak |= 1 << i;
-            L[i][i] = 1.0;
-            for (int t = 0; t < i; ++t) L[i][t] = 0.0;
-          } else {
-            L[i][i] = sqrt(sum);
-          }
-        } else {
-          L[i][j] = (weak >> i & 1) ? 0.0 : sum / L[j][j];
-        }
-      }
-    const int proj = weak | badmask;  // columns that are only projected
     // R = D L^{-T} on the healthy columns, e_j on the others (upper triangular)
-    for (int j = 0; j < b; ++j) {
-      for (int i = 0; i < b; ++i) R[i][j] = 0.0;
-      if (proj >> j & 1) {
-        R[j][j] = 1.0;
-        continue;
-      }
+    if (row) {
       double x[kMaxB];
-      for (int i = b - 1; i >= 0; --i) {
-        if (proj >> i & 1) {
-          x[i] = 0.0;
-          continue;
-        }
-        double r = i == j ? 1.0 : 0.0;
-        for (int k = i + 1; k < b; ++k) r -= L[k][i] * x[k];
+#pragma unroll
+      for (int i = kMaxB - 1; i >= 0; --i) {
+        x[i] = 0.0;
+        if (i >= b || (proj >> i & 1) || (proj >> tid & 1)) continue;
+        double r = i == tid ? 1.0 : 0.0;
+#pragma unroll
+        for (int k = i + 1; k < kMaxB; ++k)
+          if (k < b) r -= L[k][i] * x[k];
         x[i] = r / L[i][i];
       }
-      for (int i = 0; i < b; ++i) R[i][j] = d[i] * x[i];
+#pragma unroll
+      for (int i = 0; i < kMaxB; ++i)
+        if (i < b) R[i][tid] = proj >> tid & 1 ? (i == tid ? 1.0 : 0.0) : d[i] * x[i];
     }
-    bmask = badmask;
+    if (tid == 0) bad[q] = badmask;
   }
   __syncthreads();
   double* c = M + size_t(q) * (kMaxLim * kMaxB);
@@ -812,7 +802,6 @@ __global__ void __launch_bounds__(64) k_bpip(int Q, int c0, int b, const double*
     }
     c[k * kMaxB + j] = v;
   }
-  if (tid == 0) bad[q] = bmask;
 }
 
 template <class T>
