@@ -39,7 +39,9 @@ namespace {
 constexpr int kDense = 64;     // problems up to this dimension are solved exactly
 constexpr int kJac = 64;       // largest matrix of the batched Jacobi
 constexpr int kChunk = 64;     // rows summed in the working precision before an FP64 add
-constexpr int kTile = 16 * kChunk;  // rows of one problem per CTA of the segmented products
+// rows of one problem per CTA of the segmented products (24 problems of 105,000
+// rows together: 1024 rows left a third of the SMs without a CTA)
+constexpr int kTile = 8 * kChunk;
 constexpr int kMaxB = 8;       // block size limit
 constexpr int kMaxLim = 40;    // basis limit
 
@@ -86,10 +88,12 @@ constexpr size_t jac_smem() {
 // left to rotate away.  kprev = k takes Zout as approximate eigenvectors of
 // the whole matrix (from the FP32 solve of the same A).
 template <class R>
-__global__ void __launch_bounds__(256) k_bjacobi(const double* __restrict__ Ain, const int* __restrict__ kdim,
-                                                 int kconst, double* __restrict__ w, double* Zout,
-                                                 const int* __restrict__ fz, int kprev, int ortho,
-                                                 const int* __restrict__ solved) {
+constexpr int kJacThreads = sizeof(R) == 4 ? 1024 : 256;
+
+template <class R>
+__global__ void __launch_bounds__(kJacThreads<R>)
+    k_bjacobi(const double* __restrict__ Ain, const int* __restrict__ kdim, int kconst, double* __restrict__ w,
+              double* Zout, const int* __restrict__ fz, int kprev, int ortho, const int* __restrict__ solved) {
   constexpr R kConv = sizeof(R) == 4 ? R(1e-12) : R(1e-24);   // (off / total)^2 at convergence
   constexpr R kTiny = sizeof(R) == 4 ? R(1e-30) : R(1e-300);
   constexpr R kSkip = sizeof(R) == 4 ? R(1e-7) : R(1e-17);
@@ -189,21 +193,21 @@ __global__ void __launch_bounds__(256) k_bjacobi(const double* __restrict__ Ain,
       tot += v;
       if (r != c) off += v;
     }
-    // warp sums, then the 8 warps' in a fixed order
+    // warp sums, then the warps' in a fixed order
     for (int o = 16; o; o >>= 1) {
       off += __shfl_xor_sync(0xffffffffu, off, o);
       tot += __shfl_xor_sync(0xffffffffu, tot, o);
     }
     if ((tid & 31) == 0) {
       red[tid >> 5] = off;
-      red[8 + (tid >> 5)] = tot;
+      red[32 + (tid >> 5)] = tot;
     }
     __syncthreads();
     if (tid == 0) {
       R offs = 0, tots = 0;
-      for (int w8 = 0; w8 < int(blockDim.x >> 5); ++w8) {
+      for (int w8 = 0; w8 < kJacThreads<R> / 32; ++w8) {
         offs += red[w8];
-        tots += red[8 + w8];
+        tots += red[32 + w8];
       }
       done = offs <= kConv * tots || offs == R(0);
     }
@@ -417,7 +421,9 @@ __global__ void __launch_bounds__(256) k_brefine(const double* __restrict__ Ain,
 // a 64-row chunk, chunks in FP64.  FP64 engine: double-float products (FP64
 // operands split once into FP32 pairs) summed over a 32-row chunk, chunks in
 // FP64.  The 8 warps are added in a fixed order.
-template <class T>
+// HI: K > 32, lanes own a second column (without: 35 -> 16 us in FP32, 162 -> 57
+// in FP64, together with the smaller tile).
+template <class T, bool HI>
 __global__ void __launch_bounds__(256) k_bxty(const BatchChunk* __restrict__ tiles, const T* __restrict__ X, int ldx,
                                               int xo, int K, const T* __restrict__ Y, int ldy, int yo, int J,
                                               double* __restrict__ part, const int* __restrict__ fz) {
@@ -429,7 +435,7 @@ __global__ void __launch_bounds__(256) k_bxty(const BatchChunk* __restrict__ til
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const BatchChunk tl = tiles[blockIdx.x];
   if (fz[tl.prob]) return;
-  const bool a0 = lane < K, a1 = lane + 32 < K;
+  const bool a0 = lane < K, a1 = HI && lane + 32 < K;
   double d0[kMaxB], d1[kMaxB];
 #pragma unroll
   for (int j = 0; j < kMaxB; ++j) { d0[j] = 0.0; d1[j] = 0.0; }
@@ -473,7 +479,7 @@ __global__ void __launch_bounds__(256) k_bxty(const BatchChunk* __restrict__ til
 #pragma unroll
           for (int j = 0; j < kMaxB; ++j) {
             sh0[j] = fmaf(float(xa[u]), yr[j], sh0[j]);
-            sh1[j] = fmaf(float(xb[u]), yr[j], sh1[j]);
+            if constexpr (HI) sh1[j] = fmaf(float(xb[u]), yr[j], sh1[j]);
           }
         }
       }
@@ -481,7 +487,7 @@ __global__ void __launch_bounds__(256) k_bxty(const BatchChunk* __restrict__ til
 #pragma unroll
     for (int j = 0; j < kMaxB; ++j) {
       d0[j] += double(sh0[j]) + double(sl0[j]);
-      d1[j] += double(sh1[j]) + double(sl1[j]);
+      if constexpr (HI) d1[j] += double(sh1[j]) + double(sl1[j]);
     }
   }
 #pragma unroll
@@ -498,14 +504,22 @@ __global__ void __launch_bounds__(256) k_bxty(const BatchChunk* __restrict__ til
   }
 }
 
-// G[q][K x J] = sum of the partials of problem q's chunks, in chunk order
-__global__ void k_breduce(const uint32_t* __restrict__ pchunk, const double* __restrict__ part, int K, int J,
-                          double* __restrict__ G, const int* __restrict__ fz) {
-  const int q = blockIdx.x;
+// G = sum of a problem's tile partials: 32 outputs a CTA, warp w adds every 8th
+// tile, the 8 warps are added in a fixed order (one CTA a problem: 10 us; 5).
+__global__ void __launch_bounds__(256) k_breduce(const uint32_t* __restrict__ pchunk, const double* __restrict__ part,
+                                                 int n, double* __restrict__ G, const int* __restrict__ fz) {
+  __shared__ double red[8][32];
+  const int q = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31, o = blockIdx.y * 32 + lane;
   if (fz[q]) return;
-  for (int o = threadIdx.x; o < K * J; o += blockDim.x) {
-    double s = 0.0;
-    for (uint32_t c = pchunk[q]; c < pchunk[q + 1]; ++c) s += part[size_t(c) * (kMaxLim * kMaxB) + o];
+  const uint32_t c1 = pchunk[q + 1];
+  double s = 0.0;
+  if (o < n)
+#pragma unroll 4
+    for (uint32_t c = pchunk[q] + w; c < c1; c += 8) s += part[size_t(c) * (kMaxLim * kMaxB) + o];
+  red[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && o < n) {
+    for (int i = 1; i < 8; ++i) s += red[i][lane];
     G[size_t(q) * (kMaxLim * kMaxB) + o] = s;
   }
 }
@@ -529,15 +543,16 @@ __global__ void k_bset_proj(int K, int J, int c0, const double* __restrict__ G, 
 // Y[r][yo + j] = beta * Y[r][yo + j] + alpha * sum_i X[r][xo + i] M[q][i][j]  (M ld mld, per problem),
 // computed in T.  One CTA per tile (rows of one problem, M staged in shared
 // memory), one thread per row: the row is read completely before it is
-// written (in-place safe).
-template <class T>
+// written (in-place safe).  MJ accumulators: predicated off beyond J, they still
+// cost an instruction each (J = 8: 55 us with 40, 16 us with 8).
+template <class T, int MJ>
 __global__ void __launch_bounds__(256) k_bgemm(const BatchChunk* __restrict__ tiles, const T* X, int ldx, int xo,
                                                int K, const double* __restrict__ M, size_t mstride, int mld, T* Y,
                                                int ldy, int yo, int J, double alpha, double beta,
                                                const int* __restrict__ fz) {
   constexpr bool DF = sizeof(T) == 8;  // FP64 engine: double-float arithmetic
-  __shared__ float Mh[kMaxLim * kMaxLim];
-  __shared__ float Ml[DF ? kMaxLim * kMaxLim : 1];
+  __shared__ float Mh[kMaxLim * MJ];
+  __shared__ float Ml[DF ? kMaxLim * MJ : 1];
   const BatchChunk tl = tiles[blockIdx.x];
   if (fz[tl.prob]) return;
   const double* Mq = M + size_t(tl.prob) * mstride;
@@ -548,27 +563,27 @@ __global__ void __launch_bounds__(256) k_bgemm(const BatchChunk* __restrict__ ti
   }
   __syncthreads();
   for (uint32_t r = tl.row0 + threadIdx.x; r < tl.row1; r += blockDim.x) {
-    float ah[kMaxLim], al[kMaxLim];
+    float ah[MJ], al[MJ];
 #pragma unroll
-    for (int j = 0; j < kMaxLim; ++j) { ah[j] = 0.f; al[j] = 0.f; }
+    for (int j = 0; j < MJ; ++j) { ah[j] = 0.f; al[j] = 0.f; }
     const T* xr = X + size_t(r) * ldx + xo;
     for (int i = 0; i < K; ++i) {
       if constexpr (DF) {
         float xh, xl;
         df_split(double(xr[i]), xh, xl);
 #pragma unroll
-        for (int j = 0; j < kMaxLim; ++j)
+        for (int j = 0; j < MJ; ++j)
           if (j < J) df_mac(ah[j], al[j], xh, xl, Mh[i * J + j], Ml[i * J + j]);
       } else {
         const float xv = float(xr[i]);
 #pragma unroll
-        for (int j = 0; j < kMaxLim; ++j)
+        for (int j = 0; j < MJ; ++j)
           if (j < J) ah[j] = fmaf(xv, Mh[i * J + j], ah[j]);
       }
     }
     T* yr = Y + size_t(r) * ldy + yo;
 #pragma unroll
-    for (int j = 0; j < kMaxLim; ++j)
+    for (int j = 0; j < MJ; ++j)
       if (j < J) {
         const T v = DF ? T(double(ah[j]) + double(al[j])) : T(ah[j]);
         yr[j] = beta == 0.0 ? v : T(beta) * yr[j] + v;
@@ -910,13 +925,21 @@ struct BEngine {
 
   // G[q] = X[:, xo:xo+K]^T Y[:, yo:yo+J] per (unfrozen) problem
   void xty(const T* X, int ldx, int xo, int K, const T* Y, int ldy, int yo, int J) {
-    k_bxty<T><<<unsigned(bs.nchunks), 256, 0, s>>>(bs.chunks.p, X, ldx, xo, K, Y, ldy, yo, J, part.p, fz.p);
-    k_breduce<<<Q, 128, 0, s>>>(bs.pchunk.p, part.p, K, J, G.p, fz.p);
+    auto go = [&](auto kern) {
+      kern<<<unsigned(bs.nchunks), 256, 0, s>>>(bs.chunks.p, X, ldx, xo, K, Y, ldy, yo, J, part.p, fz.p);
+    };
+    if (K <= 32) go(k_bxty<T, false>);
+    else go(k_bxty<T, true>);
+    k_breduce<<<dim3(unsigned(Q), unsigned(K * J + 31) / 32), 256, 0, s>>>(bs.pchunk.p, part.p, K * J, G.p, fz.p);
   }
   void gemm(const T* X, int ldx, int xo, int K, const double* Mm, size_t mstride, int mld, T* Y, int ldy, int yo,
             int J, double alpha, double beta) {
-    k_bgemm<T><<<unsigned(bs.nchunks), 256, 0, s>>>(bs.chunks.p, X, ldx, xo, K, Mm, mstride, mld, Y, ldy, yo, J,
-                                                     alpha, beta, fz.p);
+    auto go = [&](auto kern) {
+      kern<<<unsigned(bs.nchunks), 256, 0, s>>>(bs.chunks.p, X, ldx, xo, K, Mm, mstride, mld, Y, ldy, yo, J, alpha,
+                                                beta, fz.p);
+    };
+    if (J <= kMaxB) go(k_bgemm<T, kMaxB>);
+    else go(k_bgemm<T, kMaxLim>);
   }
   void spmm(int c0) {
     if constexpr (sizeof(T) == 4) {
@@ -964,15 +987,12 @@ struct BEngine {
     k_bset_proj<<<Q, 128, 0, s>>>(k, b, k - b, G.p, S.p, fz.p);
     // warm start from the previous step's eigenvectors (size k - b; after a
     // restart the kept block is diagonal and Z's leading block the identity).
-    // FP32 phase: FP32 sweeps, their vectors refined to FP64; FP64 sweeps only
-    // where the refinement did not converge
-    if (sizeof(T) == 4) {
-      k_bjacobi<float><<<Q, 256, jac_smem<float>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0, nullptr);
-      refine(k);
-      k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k, 1, solved.p);
-    } else {
-      k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0, nullptr);
-    }
+    // FP32 sweeps, their vectors refined to FP64; FP64 sweeps only where the
+    // refinement did not converge
+    k_bjacobi<float><<<Q, kJacThreads<float>, jac_smem<float>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k - b, 0,
+                                                                       nullptr);
+    refine(k);
+    k_bjacobi<double><<<Q, 256, jac_smem<double>(), s>>>(S.p, nullptr, k, w.p, Z.p, fz.p, k, 1, solved.p);
     k_bresid<T><<<unsigned(bs.nchunks), 256, 0, s>>>(bs.chunks.p, V.p, AV.p, lim, k, w.p, Z.p, R.p, 8, b, fz.p);
     xty(R.p, 8, 0, b, R.p, 8, 0, b);
     k_bconv<<<1, 256, 0, s>>>(Q, nev, b, G.p, tol, rnorm.p, fz.p, kfreeze.p, k, nconv.p);
