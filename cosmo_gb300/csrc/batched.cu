@@ -75,7 +75,9 @@ __global__ void k_dense_fill(int n, uint64_t r0, const uint64_t* __restrict__ rp
 // FP64 (k_brefine); the FP64 Jacobi takes the matrices where that fails, from
 // the FP32 vectors (re-orthonormalized: ortho).  Cyclic Jacobi with the round-robin ordering: each round
 // applies k/2 disjoint rotations at once, skipping those whose |a_pq| is
-// below 1e-17 (FP32: 1e-7) of sqrt|a_pp a_qq|; at most 40 sweeps.
+// below 1e-17 (FP32: 1e-7) of sqrt|a_pp a_qq|; at most 40 sweeps.  FP32, k up
+// to 40: bound by the latency of a round, 231 us with 256 threads in a row over
+// blocks and rows, 181 with 1024, 160 with a warp a row (512 threads 174).
 template <class R>
 constexpr size_t jac_smem() {
   return (size_t(3) * kJac * (kJac + 1) + 256 + kJac) * sizeof(R) + (2 * kJac + 8) * sizeof(int);
@@ -87,6 +89,12 @@ constexpr size_t jac_smem() {
 // already diagonal, with Z = P, so only the coupling to the newest rows is
 // left to rotate away.  kprev = k takes Zout as approximate eigenvectors of
 // the whole matrix (from the FP32 solve of the same A).
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 template <class R>
 constexpr int kJacThreads = sizeof(R) == 4 ? 1024 : 256;
 
@@ -222,7 +230,15 @@ __global__ void __launch_bounds__(kJacThreads<R>)
         R c = 1, s = 0;
         if (q < k) {
           const R apq = A[p][q];
-          if (fabs(apq) > kTiny && fabs(apq) > kSkip * sqrt(fabs(A[p][p] * A[q][q]))) {
+          if constexpr (sizeof(R) == 4) {
+            // approximate roots: c^2 + s^2 = 1 to FP32 rounding, and the vectors are refined
+            if (fabsf(apq) > kTiny && apq * apq > kSkip * kSkip * fabsf(A[p][p] * A[q][q])) {
+              const float tau = __fdividef(A[q][q] - A[p][p], 2.f * apq);
+              const float t = copysignf(__fdividef(1.f, fabsf(tau) + sqrt_approx(1.f + tau * tau)), tau);
+              c = rsqrtf(1.f + t * t);
+              s = t * c;
+            }
+          } else if (fabs(apq) > kTiny && fabs(apq) > kSkip * sqrt(fabs(A[p][p] * A[q][q]))) {
             const R tau = (A[q][q] - A[p][p]) / (R(2) * apq);
             const R t = (tau >= 0 ? R(1) : R(-1)) / (fabs(tau) + sqrt(R(1) + tau * tau));
             c = R(1) / sqrt(R(1) + t * t);
@@ -240,31 +256,44 @@ __global__ void __launch_bounds__(kJacThreads<R>)
       // pair b columns) is rotated from both sides by one thread; the rows of
       // Z's column pairs go to the threads after the blocks
       const int np2 = kk / 2;
-      for (int i = tid; i < np2 * np2 + k * np2; i += blockDim.x) {
-        if (i < np2 * np2) {
-          const int a = i / np2, bb = i - a * np2;
-          const int pa = rp[a], qa = rq[a], pb = rp[bb], qb = rq[bb];
-          const bool va = qa < k, vb = qb < k;
-          const R ca = rc[a], sa = rs[a], cb = rc[bb], sb = rs[bb];
-          if ((sa == R(0)) && (sb == R(0))) continue;
-          const R x00 = A[pa][pb], x01 = vb ? A[pa][qb] : R(0);
-          const R x10 = va ? A[qa][pb] : R(0), x11 = (va && vb) ? A[qa][qb] : R(0);
-          // rows p, q of the block: J_a^T
-          const R y00 = ca * x00 - sa * x10, y01 = ca * x01 - sa * x11;
-          const R y10 = sa * x00 + ca * x10, y11 = sa * x01 + ca * x11;
-          // columns p, q: J_b
-          A[pa][pb] = cb * y00 - sb * y01;
-          if (vb) A[pa][qb] = sb * y00 + cb * y01;
-          if (va) A[qa][pb] = cb * y10 - sb * y11;
-          if (va && vb) A[qa][qb] = sb * y10 + cb * y11;
-        } else {
-          const int t = i - np2 * np2, bb = t / k, r = t - bb * k;
-          const int pb = rp[bb], qb = rq[bb];
-          const R cb = rc[bb], sb = rs[bb];
-          if (qb >= k || sb == R(0)) continue;
-          const R zp = Z[r][pb], zq = Z[r][qb];
-          Z[r][pb] = cb * zp - sb * zq;
-          Z[r][qb] = sb * zp + cb * zq;
+      // FP32: a warp takes the blocks of a pair a, or a row of Z, with its
+      // lanes on the pairs bb (bound by latency); FP64: threads in a row over
+      // all of them (bound by the pipe, which idle lanes cost as much)
+      const auto block = [&](int a, int bb) {
+        const int pa = rp[a], qa = rq[a], pb = rp[bb], qb = rq[bb];
+        const bool va = qa < k, vb = qb < k;
+        const R ca = rc[a], sa = rs[a], cb = rc[bb], sb = rs[bb];
+        if ((sa == R(0)) && (sb == R(0))) return;
+        const R x00 = A[pa][pb], x01 = vb ? A[pa][qb] : R(0);
+        const R x10 = va ? A[qa][pb] : R(0), x11 = (va && vb) ? A[qa][qb] : R(0);
+        // rows p, q of the block: J_a^T
+        const R y00 = ca * x00 - sa * x10, y01 = ca * x01 - sa * x11;
+        const R y10 = sa * x00 + ca * x10, y11 = sa * x01 + ca * x11;
+        // columns p, q: J_b
+        A[pa][pb] = cb * y00 - sb * y01;
+        if (vb) A[pa][qb] = sb * y00 + cb * y01;
+        if (va) A[qa][pb] = cb * y10 - sb * y11;
+        if (va && vb) A[qa][qb] = sb * y10 + cb * y11;
+      };
+      const auto zrow = [&](int r, int bb) {
+        const int pb = rp[bb], qb = rq[bb];
+        const R cb = rc[bb], sb = rs[bb];
+        if (qb >= k || sb == R(0)) return;
+        const R zp = Z[r][pb], zq = Z[r][qb];
+        Z[r][pb] = cb * zp - sb * zq;
+        Z[r][qb] = sb * zp + cb * zq;
+      };
+      if constexpr (sizeof(R) == 4) {
+        const int lane = tid & 31;
+        if (lane < np2)
+          for (int t = tid >> 5; t < np2 + k; t += kJacThreads<R> / 32) {
+            if (t < np2) block(t, lane);
+            else zrow(t - np2, lane);
+          }
+      } else {
+        for (int i = tid; i < np2 * np2 + k * np2; i += kJacThreads<R>) {
+          if (i < np2 * np2) block(i / np2, i % np2);
+          else zrow((i - np2 * np2) % k, (i - np2 * np2) / k);
         }
       }
       __syncthreads();
@@ -544,7 +573,7 @@ __global__ void k_bset_proj(int K, int J, int c0, const double* __restrict__ G, 
 // computed in T.  One CTA per tile (rows of one problem, M staged in shared
 // memory), one thread per row: the row is read completely before it is
 // written (in-place safe).  MJ accumulators: predicated off beyond J, they still
-// cost an instruction each (J = 8: 55 us with 40, 16 us with 8).
+// cost an instruction each (J = 8: 55 us with 40, 16 us with 8; J = 16: 53 and 28).
 template <class T, int MJ>
 __global__ void __launch_bounds__(256) k_bgemm(const BatchChunk* __restrict__ tiles, const T* X, int ldx, int xo,
                                                int K, const double* __restrict__ M, size_t mstride, int mld, T* Y,
@@ -738,7 +767,7 @@ __global__ void __launch_bounds__(64) k_bpip(int Q, int c0, int b, const double*
   // one CTA of 64 threads per problem: the b x b Gram correction and the
   // (c0 + b) x b coefficients by all, the factorisation by one lane per row and
   // the triangular solves by one lane per column.  Bound by the latency of FP64
-  // square roots and divisions (80 us when one thread did them all; 24 us).
+  // square roots (80 us when one thread did them all, 24 with divisions; 15 us).
   const int q = blockIdx.x, tid = threadIdx.x;
   if (q >= Q) return;
   if (fz[q]) {
@@ -778,9 +807,9 @@ __global__ void __launch_bounds__(64) k_bpip(int Q, int c0, int b, const double*
         for (int t = 0; t < j; ++t) sum -= L[tid][t] * L[j][t];
       // numerically dependent on the columns before: project only
       if (__ballot_sync(all, tid == j && live && !(sum > 1e-24))) proj |= 1 << j;
-      if (tid == j) L[j][j] = proj >> j & 1 ? 1.0 : sqrt(sum);
+      if (tid == j) L[j][j] = proj >> j & 1 ? 1.0 : rsqrt(sum);  // the reciprocal: nothing else is used
       __syncwarp();
-      if (row && tid > j) L[tid][j] = live && !(proj >> j & 1) ? sum / L[j][j] : 0.0;
+      if (row && tid > j) L[tid][j] = live && !(proj >> j & 1) ? sum * L[j][j] : 0.0;
       if (tid == j && (proj >> j & 1))
         for (int t = 0; t < j; ++t) L[j][t] = 0.0;
       __syncwarp();
@@ -796,7 +825,7 @@ __global__ void __launch_bounds__(64) k_bpip(int Q, int c0, int b, const double*
 #pragma unroll
         for (int k = i + 1; k < kMaxB; ++k)
           if (k < b) r -= L[k][i] * x[k];
-        x[i] = r / L[i][i];
+        x[i] = r * L[i][i];
       }
 #pragma unroll
       for (int i = 0; i < kMaxB; ++i)
@@ -939,6 +968,7 @@ struct BEngine {
                                                 beta, fz.p);
     };
     if (J <= kMaxB) go(k_bgemm<T, kMaxB>);
+    else if (J <= 16) go(k_bgemm<T, 16>);  // the default restart
     else go(k_bgemm<T, kMaxLim>);
   }
   void spmm(int c0) {
