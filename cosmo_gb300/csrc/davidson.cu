@@ -250,17 +250,28 @@ __global__ void __launch_bounds__(256) k_xty_df(uint64_t n, const double* __rest
     float c0h[JMAX], c0l[JMAX], c1h[JMAX], c1l[JMAX];
 #pragma unroll
     for (int j = 0; j < JMAX; ++j) { c0h[j] = c0l[j] = c1h[j] = c1l[j] = 0.f; }
-    for (int rr = 0; rr < rows; ++rr) {
-      const double* xr = X + (c0 + rr) * ldx + xo;
-      float xah = 0.f, xal = 0.f, xbh = 0.f, xbl = 0.f;
-      if (a0) df_split(xr[lane], xah, xal);
-      if (a1) df_split(xr[lane + 32], xbh, xbl);
-      const float* yhr = yh[wl] + rr * JMAX;
-      const float* ylr = yl[wl] + rr * JMAX;
+    constexpr int U = 4;  // rows of X loads in flight per lane
+    for (int rr = 0; rr < rows; rr += U) {
+      double xa[U], xb[U];
 #pragma unroll
-      for (int j = 0; j < JMAX; ++j) {
-        df_mac(c0h[j], c0l[j], xah, xal, yhr[j], ylr[j]);
-        if (a1) df_mac(c1h[j], c1l[j], xbh, xbl, yhr[j], ylr[j]);
+      for (int u = 0; u < U; ++u) {
+        const double* xr = X + (c0 + rr + u) * ldx + xo;
+        const bool ok = rr + u < rows;
+        xa[u] = a0 && ok ? xr[lane] : 0.0;
+        xb[u] = a1 && ok ? xr[lane + 32] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float xah, xal, xbh, xbl;
+        df_split(xa[u], xah, xal);
+        df_split(xb[u], xbh, xbl);
+        const float* yhr = yh[wl] + (rr + u) * JMAX;
+        const float* ylr = yl[wl] + (rr + u) * JMAX;
+#pragma unroll
+        for (int j = 0; j < JMAX; ++j) {
+          df_mac(c0h[j], c0l[j], xah, xal, yhr[j], ylr[j]);
+          if (a1) df_mac(c1h[j], c1l[j], xbh, xbl, yhr[j], ylr[j]);
+        }
       }
     }
 #pragma unroll
@@ -279,14 +290,24 @@ __global__ void __launch_bounds__(256) k_xty_df(uint64_t n, const double* __rest
   }
 }
 
+// 32-byte load of 4 consecutive doubles (32-byte aligned address); coherent, as
+// the gemm may write the rows it reads
+__device__ __forceinline__ void ld4c(const double* p, double (&v)[4]) {
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+               : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+               : "l"(p)
+               : "memory");
+}
+
 // R = AB s_c - lam_c B s_c of the FP64 engine in double-float, one thread per
-// row; s and lam as FP32 pairs in shared memory; R and the norms in FP64.
+// row, read 4 values (32 bytes) at a time when aligned; s and lam as FP32 pairs in shared memory; R and the norms in FP64.
 template <int CMAX, int KM>
 __global__ void __launch_bounds__(256) k_resid_df(uint64_t n, const double* __restrict__ B,
                                                   const double* __restrict__ AB, int ld, int K,
                                                   const double* __restrict__ Sc, const double* __restrict__ lam, int C,
-                                                  double* __restrict__ R, int ldr, double* __restrict__ part) {
-  __shared__ float sh_[KM * CMAX], sl_[KM * CMAX];
+                                                  double* __restrict__ R, int ldr, double* __restrict__ part,
+                                                  bool vec) {
+  __shared__ __align__(16) float sh_[KM * CMAX], sl_[KM * CMAX];
   __shared__ double ls[CMAX];
   __shared__ double red[8][CMAX];
   for (int i = threadIdx.x; i < KM * CMAX; i += blockDim.x) {
@@ -304,17 +325,27 @@ __global__ void __launch_bounds__(256) k_resid_df(uint64_t n, const double* __re
     for (int c = 0; c < CMAX; ++c) { ah[c] = al[c] = bh[c] = bl[c] = 0.f; }
     const double* br = B + r * ld;
     const double* abr = AB + r * ld;
-    for (int k = 0; k < K; ++k) {
+    const auto add = [&](int k, double bv, double av) {
       float xbh, xbl, xah, xal;
-      df_split(br[k], xbh, xbl);
-      df_split(abr[k], xah, xal);
+      df_split(bv, xbh, xbl);
+      df_split(av, xah, xal);
 #pragma unroll
       for (int c = 0; c < CMAX; ++c) {
         const float s0 = sh_[k * CMAX + c], s1 = sl_[k * CMAX + c];
         df_mac(ah[c], al[c], xah, xal, s0, s1);
         df_mac(bh[c], bl[c], xbh, xbl, s0, s1);
       }
-    }
+    };
+    int k = 0;
+    if (vec)
+      for (; k + 4 <= K; k += 4) {
+        double bv[4], av[4];
+        ld4c(br + k, bv);
+        ld4c(abr + k, av);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) add(k + u, bv[u], av[u]);
+      }
+    for (; k < K; ++k) add(k, br[k], abr[k]);
 #pragma unroll
     for (int c = 0; c < CMAX; ++c)
       if (c < C) {
@@ -344,8 +375,8 @@ __global__ void __launch_bounds__(256) k_resid_df(uint64_t n, const double* __re
 template <int JMAX, int KM>
 __global__ void __launch_bounds__(256) k_gemm_df(uint64_t n, const double* X, int ldx, int xo, int K,
                                                  const double* __restrict__ G, double* Y, int ldy, int yo, int J,
-                                                 double alpha, double beta) {
-  __shared__ float gh[KM * JMAX], gl[KM * JMAX];
+                                                 double alpha, double beta, bool vec) {
+  __shared__ __align__(16) float gh[KM * JMAX], gl[KM * JMAX];
   for (int i = threadIdx.x; i < KM * JMAX; i += blockDim.x) {
     const int k = i / JMAX, j = i % JMAX;
     df_split((k < K && j < J) ? alpha * G[k * J + j] : 0.0, gh[i], gl[i]);
@@ -356,12 +387,21 @@ __global__ void __launch_bounds__(256) k_gemm_df(uint64_t n, const double* X, in
 #pragma unroll
     for (int j = 0; j < JMAX; ++j) { ah[j] = 0.f; al[j] = 0.f; }
     const double* xr = X + r * ldx + xo;
-    for (int k = 0; k < K; ++k) {
+    const auto add = [&](int k, double xv) {
       float xh, xl;
-      df_split(xr[k], xh, xl);
+      df_split(xv, xh, xl);
 #pragma unroll
       for (int j = 0; j < JMAX; ++j) df_mac(ah[j], al[j], xh, xl, gh[k * JMAX + j], gl[k * JMAX + j]);
-    }
+    };
+    int k = 0;
+    if (vec)
+      for (; k + 4 <= K; k += 4) {
+        double xv[4];
+        ld4c(xr + k, xv);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) add(k + u, xv[u]);
+      }
+    for (; k < K; ++k) add(k, xr[k]);
     double* yr = Y + r * ldy + yo;
 #pragma unroll
     for (int j = 0; j < JMAX; ++j)
@@ -894,7 +934,7 @@ struct Engine {
     nume = c.nume;
     lim = c.lim;
     mblock = c.block;
-    int align = sizeof(T) == 4 ? 4 : 2;
+    const int align = 4;  // FP64: rows of whole 32-byte loads
     L = (lim + align - 1) / align * align;
     if (lim > kMaxLim) throw Error(CG_ERR_ARG, "lim above 128 is not supported");
     if (mblock > kMaxC || nume > kMaxC) throw Error(CG_ERR_ARG, "block and nstates must be <= 16");
@@ -1015,7 +1055,8 @@ struct Engine {
       if (J <= 32 && J >= 3 && cfg.spmm_prec == CG_PREC_REFINE) {
         const double* Xd = reinterpret_cast<const double*>(Xp);
         double* Yd = reinterpret_cast<double*>(Yp);
-#define CG_GEMM_DF(JM, KM) k_gemm_df<JM, KM><<<grid, 256, 0, s>>>(n, Xd, L, xo, K, small2.p, Yd, ldy, yo, J, alpha, beta)
+        const bool v4 = reinterpret_cast<uintptr_t>(Xp + xo) % 32 == 0 && L % 4 == 0;
+#define CG_GEMM_DF(JM, KM) k_gemm_df<JM, KM><<<grid, 256, 0, s>>>(n, Xd, L, xo, K, small2.p, Yd, ldy, yo, J, alpha, beta, v4)
         if (J <= 8) { if (wide) CG_GEMM_DF(8, kMaxLim); else CG_GEMM_DF(8, kMaxK); }
         else if (J <= 16) { if (wide) CG_GEMM_DF(16, kMaxLim); else CG_GEMM_DF(16, kMaxK); }
         else { if (wide) CG_GEMM_DF(32, kMaxLim); else CG_GEMM_DF(32, kMaxK); }
@@ -1202,7 +1243,9 @@ struct Engine {
     bool done = false;
     if constexpr (sizeof(T) == 8) {
       if (cfg.spmm_prec == CG_PREC_REFINE) {
-#define CG_RESID_DF(CM, KM) k_resid_df<CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam.p, C, R.p, ldr, part.p)
+        const bool v4 = L % 4 == 0 && reinterpret_cast<uintptr_t>(B.p) % 32 == 0 &&
+                        reinterpret_cast<uintptr_t>(AB.p) % 32 == 0;
+#define CG_RESID_DF(CM, KM) k_resid_df<CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam.p, C, R.p, ldr, part.p, v4)
         if (C <= 8) { if (kpass > kMaxK) CG_RESID_DF(8, kMaxLim); else CG_RESID_DF(8, kMaxK); }
         else { if (kpass > kMaxK) CG_RESID_DF(16, kMaxLim); else CG_RESID_DF(16, kMaxK); }
 #undef CG_RESID_DF

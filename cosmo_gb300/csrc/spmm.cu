@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "device.h"
+#include "dfloat.h"
 #include "factored.h"
 #include "tiled.h"
 #include "virtual.h"
@@ -398,9 +399,7 @@ __global__ void k_stage_df(uint64_t n, const double* __restrict__ x, int ldx, in
   uint64_t i = idx / NV;
   int j = int(idx % NV);
   double v = j < m ? x[i * ldx + j] : 0.0;
-  float h = float(v);
-  w[i * (2 * NV) + j] = h;
-  w[i * (2 * NV) + NV + j] = float(v - double(h));
+  df_split(v, w[i * (2 * NV) + j], w[i * (2 * NV) + NV + j]);
 }
 
 // one pass of NV vectors of the double-float product (m of them stored)
