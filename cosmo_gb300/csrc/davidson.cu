@@ -23,6 +23,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <numeric>
 
 #include "davidson.h"
@@ -34,188 +35,110 @@
 namespace cg {
 namespace {
 
-constexpr int kTile = 32;   // rows per tile
 constexpr int kMaxK = 64;   // basis columns per tall-skinny kernel call
 constexpr int kMaxLim = 128;  // basis limit (calls over more than kMaxK columns are split or use the 128-row forms)
 constexpr int kMaxKeep = 64;  // Ritz vectors kept at a thick restart
 constexpr int kMaxJ = 32;   // right-hand columns per call
 constexpr int kMaxC = 16;   // residual candidates per call
-constexpr int kThreads = 256;
 
-template <class T>
-__global__ void __launch_bounds__(kThreads) k_xty(uint64_t n, const T* __restrict__ X, int ldx, int xo, int K,
-                                                  const T* __restrict__ Y, int ldy, int yo, int J,
-                                                  double* __restrict__ part, uint64_t rows_per_cta) {
-  __shared__ T xs[kTile * kMaxK];
-  __shared__ T ys[kTile * kMaxJ];
-  const int nout = K * J;
-  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const uint64_t r0 = uint64_t(blockIdx.x) * rows_per_cta;
-  const uint64_t r1 = min(n, r0 + rows_per_cta);
-  for (uint64_t base = r0; base < r1; base += kTile) {
-    const int rows = int(min(uint64_t(kTile), r1 - base));
-    for (int idx = threadIdx.x; idx < kTile * K; idx += blockDim.x) {
-      int r = idx / K, k = idx - r * K;
-      xs[idx] = r < rows ? X[(base + r) * ldx + xo + k] : T(0);
-    }
-    for (int idx = threadIdx.x; idx < kTile * J; idx += blockDim.x) {
-      int r = idx / J, j = idx - r * J;
-      ys[idx] = r < rows ? Y[(base + r) * ldy + yo + j] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      int o = threadIdx.x + q * kThreads;
-      if (o < nout) {
-        int k = o / J, j = o - k * J;
-        T t = T(0);
-#pragma unroll 8
-        for (int r = 0; r < kTile; ++r) t = fma(xs[r * K + k], ys[r * J + j], t);
-        acc[q] += double(t);
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    int o = threadIdx.x + q * kThreads;
-    if (o < nout) part[uint64_t(blockIdx.x) * nout + o] = acc[q];
-  }
-}
-
-// out[o] = sum_c part[c * nout + o]: one CTA per output, strided per-thread
-// sums and a fixed-order tree, so the result is deterministic.
-__global__ void k_reduce_parts(const double* __restrict__ part, int nparts, int nout, double* __restrict__ out) {
-  __shared__ double red[128];
-  const int o = blockIdx.x;
+// out[(o / cols) * ldo + o % cols] = sum_c part[c * nout + o]: 32 outputs a CTA,
+// warp w adds every 32nd part, the warps' sums in a fixed order, so the result
+// is deterministic.  out may be pinned host memory: the copy back was an
+// operation of its own after every X^T Y.
+__global__ void __launch_bounds__(1024) k_reduce_parts(const double* __restrict__ part, int nparts, int nout,
+                                                       double* __restrict__ out, int cols, int ldo) {
+  __shared__ double red[32][33];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, o = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int c = threadIdx.x; c < nparts; c += 128) s += part[uint64_t(c) * nout + o];
-  red[threadIdx.x] = s;
+  if (o < nout)
+#pragma unroll 8
+    for (int c = w; c < nparts; c += 32) s += part[uint64_t(c) * nout + o];
+  red[w][lane] = s;
   __syncthreads();
-  for (int w = 64; w; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[o] = red[0];
+  // warp w adds up output w
+  double v = red[lane][w];
+  for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(~0u, v, d);
+  const int ow = blockIdx.x * 32 + w;
+  if (lane == 0 && ow < nout) out[(ow / cols) * ldo + ow % cols] = v;
 }
 
 // ---- streaming tall-skinny kernels -------------------------------------
-// G (K x J) partials = X[:, xo:xo+K]^T Y[:, yo:yo+J] over this CTA's rows.
-// KP = K rounded up to a power of two (<= 64) threads share one row, thread
-// k of the group owns column k of X and all J outputs of that column; FP32
-// products are summed over 64-row chunks and the chunks in FP64.
-template <class T, int JMAX>
-__global__ void __launch_bounds__(256) k_xty_s(uint64_t n, const T* __restrict__ X, int ldx, int xo, int K,
-                                               const T* __restrict__ Y, int ldy, int yo, int J, int KP,
-                                               double* __restrict__ part, uint64_t rows_per_cta) {
-  __shared__ double red[256 * 2];
-  const int k = threadIdx.x % KP, rg = threadIdx.x / KP, ngroups = 256 / KP;
-  const bool active = k < K;
-  double acc[JMAX];
-  T ch[JMAX];
+// A CTA's partial G: the sums of its 8 warps, lane l holding column l (and, in
+// rows JMAX + j, l + 32) of X, added in order.
+template <int JMAX>
+__device__ __forceinline__ void store_part(const double (*dsh)[2 * JMAX][32], int K, int J, double* __restrict__ part) {
+  __syncthreads();
+  for (int o = threadIdx.x; o < K * J; o += 256) {
+    const int k = o / J, j = o - k * J;
+    double v = 0.0;
 #pragma unroll
-  for (int j = 0; j < JMAX; ++j) { acc[j] = 0.0; ch[j] = T(0); }
-  const uint64_t r0 = uint64_t(blockIdx.x) * rows_per_cta;
-  const uint64_t r1 = min(n, r0 + rows_per_cta);
-  int cnt = 0;
-  for (uint64_t r = r0 + rg; r < r1; r += ngroups) {
-    const T xv = active ? X[r * ldx + xo + k] : T(0);
-    const T* yr = Y + r * ldy + yo;
-#pragma unroll
-    for (int j = 0; j < JMAX; ++j)
-      if (j < J) ch[j] = fma(xv, __ldg(yr + j), ch[j]);
-    if (++cnt == 64) {
-#pragma unroll
-      for (int j = 0; j < JMAX; ++j) { acc[j] += double(ch[j]); ch[j] = T(0); }
-      cnt = 0;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < JMAX; ++j) acc[j] += double(ch[j]);
-  // reduce the row groups: for each j, sum acc over rg (same k); J is uniform
-#pragma unroll
-  for (int j = 0; j < JMAX; ++j) {
-    if (j < J) {
-      red[threadIdx.x] = acc[j];
-      __syncthreads();
-      if (rg == 0 && active) {
-        double sum = 0.0;
-        for (int g = 0; g < ngroups; ++g) sum += red[g * KP + k];
-        part[uint64_t(blockIdx.x) * (K * J) + k * J + j] = sum;
-      }
-      __syncthreads();
-    }
+    for (int w = 0; w < 8; ++w) v += dsh[w][(k >> 5) * JMAX + j][k & 31];
+    part[uint64_t(blockIdx.x) * (K * J) + o] = v;
   }
 }
 
-// Warp-per-row-chunk X^T Y: lane l owns columns l and l + 32 of X (K <= 64);
-// four rows are loaded before they are used so each warp keeps several rows of
-// loads in flight.  FP32 (or FP64) products, 64-row chunks summed in FP64;
-// per-warp partials go to part[warp][k * J + j].
-template <class T, int JMAX>
-__global__ void __launch_bounds__(256) k_xty_w(uint64_t n, const T* __restrict__ X, int ldx, int xo, int K,
-                                               const T* __restrict__ Y, int ldy, int yo, int J,
+// FP64 X^T Y, K <= 64, J <= 16.  Bound by the FP64 pipe, which takes 16 clocks
+// for a warp instruction however many lanes it has: the K x J outputs are dealt
+// out to the lanes in order, NT each, and both operands come from staged rows
+// (2e6 rows, 10 x 10: 0.47 ms; 3.3 with a lane per column of X, 16 outputs each).
+template <int NT>
+__global__ void __launch_bounds__(256) k_xty_p(uint64_t n, const double* __restrict__ X, int ldx, int xo, int K,
+                                               const double* __restrict__ Y, int ldy, int yo, int J,
                                                double* __restrict__ part, uint64_t rows_per_warp) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t gw = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  // Y rows as float4 when every row start is 16-byte aligned; the columns past
-  // J in the last float4 are zero-weighted below (yv beyond J only meets c0/c1
-  // of columns j >= J, which are never written out)
-  const bool vec_y = (reinterpret_cast<uintptr_t>(Y + yo) % 16 == 0) && (ldy % 4 == 0) && (J % 4 == 0);
-  const uint64_t r0 = gw * rows_per_warp;
+  constexpr int CH = 8;
+  __shared__ double xs[8][CH][kMaxK], ys[8][CH][16];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const uint64_t r0 = (uint64_t(blockIdx.x) * 8 + wl) * rows_per_warp;
   const uint64_t r1 = min(n, r0 + rows_per_warp);
-  const bool a0 = lane < K, a1 = lane + 32 < K;
-  T c0[JMAX], c1[JMAX];
-  double d0[JMAX], d1[JMAX];
+  int at[NT];  // k and j of the lane's outputs
+  double tot[NT], ch[NT];
 #pragma unroll
-  for (int j = 0; j < JMAX; ++j) { c0[j] = c1[j] = T(0); d0[j] = d1[j] = 0.0; }
+  for (int t = 0; t < NT; ++t) {
+    const int o = lane + 32 * t;
+    at[t] = o < K * J ? (o / J) << 8 | o % J : 0;
+    tot[t] = ch[t] = 0.0;
+  }
   int cnt = 0;
-  for (uint64_t r = r0; r < r1; r += 4) {
-    T x0[4], x1[4], yv[4][JMAX];
+  for (uint64_t c0 = r0; c0 < r1; c0 += CH) {
+    __syncwarp();
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const bool ok = r + u < r1;
-      const T* xr = X + (r + u) * ldx + xo;
-      x0[u] = (ok && a0) ? xr[lane] : T(0);
-      x1[u] = (ok && a1) ? xr[lane + 32] : T(0);
-      const T* yr = Y + (r + u) * ldy + yo;
-      if constexpr (sizeof(T) == 4 && JMAX % 4 == 0) {
-        if (vec_y) {  // J values of the row as 16-byte loads (broadcast across the warp)
-#pragma unroll
-          for (int j4 = 0; j4 < JMAX / 4; ++j4) {
-            const float4 v = (ok && 4 * j4 < J) ? __ldg(reinterpret_cast<const float4*>(yr) + j4)
-                                                : make_float4(0.f, 0.f, 0.f, 0.f);
-            yv[u][4 * j4] = v.x;
-            yv[u][4 * j4 + 1] = v.y;
-            yv[u][4 * j4 + 2] = v.z;
-            yv[u][4 * j4 + 3] = v.w;
-          }
-          continue;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < JMAX; ++j) yv[u][j] = (ok && j < J) ? __ldg(yr + j) : T(0);
+    for (int r = 0; r < CH; ++r) {
+      const bool ok = c0 + r < r1;
+      const double* xr = X + (c0 + r) * ldx + xo;
+      xs[wl][r][lane] = ok && lane < K ? xr[lane] : 0.0;
+      xs[wl][r][lane + 32] = ok && lane + 32 < K ? xr[lane + 32] : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int i = 0; i < CH / 2; ++i) {
+      const int r = 2 * i + (lane >> 4), j = lane & 15;
+      ys[wl][r][j] = c0 + r < r1 && j < J ? Y[(c0 + r) * ldy + yo + j] : 0.0;
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (int r = 0; r < CH; ++r)
 #pragma unroll
-      for (int j = 0; j < JMAX; ++j) {
-        c0[j] = fma(x0[u], yv[u][j], c0[j]);
-        c1[j] = fma(x1[u], yv[u][j], c1[j]);
-      }
-    cnt += 4;
-    if (cnt >= 64) {
-#pragma unroll
-      for (int j = 0; j < JMAX; ++j) { d0[j] += double(c0[j]); d1[j] += double(c1[j]); c0[j] = c1[j] = T(0); }
+      for (int t = 0; t < NT; ++t) ch[t] = fma(xs[wl][r][at[t] >> 8], ys[wl][r][at[t] & 255], ch[t]);
+    if (++cnt == 64 / CH) {  // 64-row sums
       cnt = 0;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        tot[t] += ch[t];
+        ch[t] = 0.0;
+      }
     }
   }
-  double* out = part + gw * uint64_t(K * J);
+  // the 8 warps in order
+  double(*red)[32] = reinterpret_cast<double(*)[32]>(&ys[0][0][0]);
 #pragma unroll
-  for (int j = 0; j < JMAX; ++j) {
-    if (j < J) {
-      if (a0) out[lane * J + j] = d0[j] + double(c0[j]);
-      if (a1) out[(lane + 32) * J + j] = d1[j] + double(c1[j]);
+  for (int t = 0; t < NT; ++t) {
+    __syncthreads();
+    red[wl][lane] = tot[t] + ch[t];
+    __syncthreads();
+    const int o = lane + 32 * t;
+    if (wl == 0 && o < K * J) {
+      double v = red[0][lane];
+      for (int w = 1; w < 8; ++w) v += red[w][lane];
+      part[uint64_t(blockIdx.x) * (K * J) + o] = v;
     }
   }
 }
@@ -225,7 +148,7 @@ __global__ void __launch_bounds__(256) k_xty_w(uint64_t n, const T* __restrict__
 // X^T Y of the FP64 engine in double-float: as k_xty_t, with the staged Y chunk
 // held as FP32 pairs and 32-row chunks summed in double-float, then in FP64.
 template <int JMAX>
-__global__ void __launch_bounds__(256) k_xty_df(uint64_t n, const double* __restrict__ X, int ldx, int xo, int K,
+__global__ void __launch_bounds__(256, 4) k_xty_df(uint64_t n, const double* __restrict__ X, int ldx, int xo, int K,
                                                 const double* __restrict__ Y, int ldy, int yo, int J,
                                                 double* __restrict__ part, uint64_t rows_per_warp) {
   constexpr int CH = 32;
@@ -250,7 +173,7 @@ __global__ void __launch_bounds__(256) k_xty_df(uint64_t n, const double* __rest
     float c0h[JMAX], c0l[JMAX], c1h[JMAX], c1l[JMAX];
 #pragma unroll
     for (int j = 0; j < JMAX; ++j) { c0h[j] = c0l[j] = c1h[j] = c1l[j] = 0.f; }
-    constexpr int U = 4;  // rows of X loads in flight per lane
+    constexpr int U = 2;  // rows of X loads in flight per lane
     for (int rr = 0; rr < rows; rr += U) {
       double xa[U], xb[U];
 #pragma unroll
@@ -280,14 +203,7 @@ __global__ void __launch_bounds__(256) k_xty_df(uint64_t n, const double* __rest
       dsh[wl][JMAX + j][lane] += double(c1h[j]) + double(c1l[j]);
     }
   }
-  double* out = part + gw * uint64_t(K * J);
-#pragma unroll
-  for (int j = 0; j < JMAX; ++j) {
-    if (j < J) {
-      if (a0) out[lane * J + j] = dsh[wl][j][lane];
-      if (a1) out[(lane + 32) * J + j] = dsh[wl][JMAX + j][lane];
-    }
-  }
+  store_part<JMAX>(dsh, K, J, part);
 }
 
 // 32-byte load of 4 consecutive doubles (32-byte aligned address); coherent, as
@@ -416,14 +332,14 @@ __global__ void __launch_bounds__(256) k_gemm_df(uint64_t n, const double* X, in
 // the warp first copies the chunk's J columns of Y (coalesced: lane groups of
 // J read consecutive rows), then lane l owns columns l and l + 32 of X and
 // reads the J values of a row as shared-memory broadcasts.  FP32 products are
-// summed over the chunk and the chunks in FP64; per-warp partials go to
-// part[warp][k * J + j].  Any column offset yo (no alignment needed).
-template <class T, int JMAX>
-__global__ void __launch_bounds__(256, 4) k_xty_t(uint64_t n, const T* __restrict__ X, int ldx, int xo, int K,
-                                               const T* __restrict__ Y, int ldy, int yo, int J,
+// summed over the chunk and the chunks in FP64; per-CTA partials go to
+// part[CTA][k * J + j].  Any column offset yo (no alignment needed).
+template <int JMAX>
+__global__ void __launch_bounds__(256, 4) k_xty_t(uint64_t n, const float* __restrict__ X, int ldx, int xo, int K,
+                                               const float* __restrict__ Y, int ldy, int yo, int J,
                                                double* __restrict__ part, uint64_t rows_per_warp) {
-  constexpr int CH = JMAX * sizeof(T) > 32 ? 32 : 64;  // staged rows per chunk (<= 32 KB per CTA)
-  __shared__ __align__(16) T ys[8][CH * JMAX];
+  constexpr int CH = 64;  // staged rows per chunk
+  __shared__ __align__(16) float ys[8][CH * JMAX];
   // FP64 chunk sums of lane l, column j at dsh[warp][j][l] (x0) and [JMAX + j][l] (x1)
   __shared__ double dsh[8][2 * JMAX][32];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -431,7 +347,7 @@ __global__ void __launch_bounds__(256, 4) k_xty_t(uint64_t n, const T* __restric
   const uint64_t r0 = gw * rows_per_warp;
   const uint64_t r1 = min(n, r0 + rows_per_warp);
   const bool a0 = lane < K, a1 = lane + 32 < K;
-  T* yw = ys[wl];
+  float* yw = ys[wl];
 #pragma unroll
   for (int j = 0; j < 2 * JMAX; ++j) dsh[wl][j][lane] = 0.0;
   for (uint64_t c0 = r0; c0 < r1; c0 += CH) {
@@ -439,28 +355,28 @@ __global__ void __launch_bounds__(256, 4) k_xty_t(uint64_t n, const T* __restric
     __syncwarp();
     for (int i = lane; i < CH * JMAX; i += 32) {
       const int rr = i / JMAX, j = i - rr * JMAX;
-      yw[i] = (rr < rows && j < J) ? Y[(c0 + rr) * ldy + yo + j] : T(0);
+      yw[i] = (rr < rows && j < J) ? Y[(c0 + rr) * ldy + yo + j] : 0.f;
     }
     __syncwarp();
-    T c0v[JMAX], c1v[JMAX];
+    float c0v[JMAX], c1v[JMAX];
 #pragma unroll
-    for (int j = 0; j < JMAX; ++j) { c0v[j] = T(0); c1v[j] = T(0); }
-    constexpr int U = sizeof(T) == 4 ? 8 : 4;  // rows of X loads in flight per lane
+    for (int j = 0; j < JMAX; ++j) { c0v[j] = 0.f; c1v[j] = 0.f; }
+    constexpr int U = 8;  // rows of X loads in flight per lane
     for (int rr = 0; rr < rows; rr += U) {
-      const T* xr0 = X + (c0 + rr) * ldx + xo;
-      T xa[U], xb[U];
+      const float* xr0 = X + (c0 + rr) * ldx + xo;
+      float xa[U], xb[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const bool ok = rr + u < rows;
-        xa[u] = (a0 && ok) ? xr0[u * ldx + lane] : T(0);
-        xb[u] = (a1 && ok) ? xr0[u * ldx + lane + 32] : T(0);
+        xa[u] = (a0 && ok) ? xr0[u * ldx + lane] : 0.f;
+        xb[u] = (a1 && ok) ? xr0[u * ldx + lane + 32] : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const T* ya = yw + (rr + u) * JMAX;
+        const float* ya = yw + (rr + u) * JMAX;
 #pragma unroll
         for (int j = 0; j < JMAX; ++j) {
-          const T v = ya[j];
+          const float v = ya[j];
           c0v[j] = fma(xa[u], v, c0v[j]);
           c1v[j] = fma(xb[u], v, c1v[j]);
         }
@@ -472,14 +388,7 @@ __global__ void __launch_bounds__(256, 4) k_xty_t(uint64_t n, const T* __restric
       dsh[wl][JMAX + j][lane] += double(c1v[j]);
     }
   }
-  double* out = part + gw * uint64_t(K * J);
-#pragma unroll
-  for (int j = 0; j < JMAX; ++j) {
-    if (j < J) {
-      if (a0) out[lane * J + j] = dsh[wl][j][lane];
-      if (a1) out[(lane + 32) * J + j] = dsh[wl][JMAX + j][lane];
-    }
-  }
+  store_part<JMAX>(dsh, K, J, part);
 }
 
 // 32-byte load of 8 consecutive floats (32-byte aligned address): one L1
@@ -503,7 +412,9 @@ __device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
                : "memory");
 }
 
-// R[:, c] = AB s_c - lam_c B s_c for C candidates, one thread per row with the
+// R[:, c] = AB s_c - lam_c B s_c for C <= CMAX candidates (for 10, rounding up to
+// 12 instead of 16: 2e6 rows of 96 columns 0.45 -> 0.35 ms, in double-float 1.04
+// -> 0.67), one thread per row with the
 // row read 8 values (32 bytes) at a time when aligned, s in shared memory, R
 // rows written 8 columns at a time; per-CTA partial |R[:, c]|^2 (FP32 over a
 // thread's rows, FP64 across threads, fixed order).
@@ -561,11 +472,11 @@ __global__ void __launch_bounds__(256) k_resid_v(uint64_t n, const T* __restrict
     if constexpr (sizeof(T) == 4) {
       // R rows 32-byte aligned: whole 8-column groups as one store each
 #pragma unroll
-      for (int g = 0; g < CMAX / 8; ++g)
+      for (int g = 0; g < (CMAX + 7) / 8; ++g)
         if (8 * g + 8 <= cvec) {
           float v[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) v[u] = res[8 * g + u];
+          for (int u = 0; u < 8; ++u) v[u] = 8 * g + u < CMAX ? res[8 * g + u < CMAX ? 8 * g + u : 0] : 0.f;
           st8(rr + 8 * g, v);
         }
     }
@@ -654,165 +565,33 @@ __global__ void __launch_bounds__(256) k_gemm_r(uint64_t n, const T* X, int ldx,
   }
 }
 
-// Thread per row: R[:, c] = AB s_c - lam_c B s_c for C candidates, plus
-// per-CTA partial |R[:, c]|^2 (FP32 over 16-row chunks, FP64 across).
-template <class T, int CMAX>
-__global__ void __launch_bounds__(256) k_resid_s(uint64_t n, const T* __restrict__ B, const T* __restrict__ AB,
-                                                 int ld, int K, const double* __restrict__ Sc,
-                                                 const double* __restrict__ lam, int C, T* __restrict__ R, int ldr,
-                                                 double* __restrict__ part) {
-  __shared__ T ss[64 * CMAX];
-  __shared__ T ls[CMAX];
-  __shared__ double red[256];
-  for (int i = threadIdx.x; i < K * C; i += blockDim.x) ss[(i / C) * CMAX + (i % C)] = T(Sc[i]);
-  for (int i = threadIdx.x; i < CMAX; i += blockDim.x) ls[i] = i < C ? T(lam[i]) : T(0);
-  __syncthreads();
-  double nacc[CMAX];
-  T nch[CMAX];
-#pragma unroll
-  for (int c = 0; c < CMAX; ++c) { nacc[c] = 0.0; nch[c] = T(0); }
-  int cnt = 0;
-  for (uint64_t r = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; r < n; r += uint64_t(gridDim.x) * blockDim.x) {
-    T a[CMAX], b[CMAX];
-#pragma unroll
-    for (int c = 0; c < CMAX; ++c) { a[c] = T(0); b[c] = T(0); }
-    const T* br = B + r * ld;
-    const T* abr = AB + r * ld;
-    for (int k = 0; k < K; ++k) {
-      const T bv = br[k], av = abr[k];
-#pragma unroll
-      for (int c = 0; c < CMAX; ++c) {
-        a[c] = fma(av, ss[k * CMAX + c], a[c]);
-        b[c] = fma(bv, ss[k * CMAX + c], b[c]);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < CMAX; ++c)
-      if (c < C) {
-        const T res = a[c] - ls[c] * b[c];
-        R[r * ldr + c] = res;
-        nch[c] = fma(res, res, nch[c]);
-      }
-    if (++cnt == 16) {
-#pragma unroll
-      for (int c = 0; c < CMAX; ++c) { nacc[c] += double(nch[c]); nch[c] = T(0); }
-      cnt = 0;
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < CMAX; ++c) {
-    if (c < C) {
-      red[threadIdx.x] = nacc[c] + double(nch[c]);
-      __syncthreads();
-      for (int o = 128; o; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) part[uint64_t(blockIdx.x) * C + c] = red[0];
-      __syncthreads();
-    }
-  }
-}
-
-// Y[:, yo:yo+J] = beta * Y + alpha * X[:, xo:xo+K] G  (G is K x J, FP64).
-// A CTA stages its whole row tile of X before writing, so X and Y may alias.
-template <class T>
-__global__ void __launch_bounds__(kThreads) k_rows_gemm(uint64_t n, const T* X, int ldx, int xo, int K,
-                                                        const double* __restrict__ G, T* Y, int ldy, int yo, int J,
-                                                        double alpha, double beta) {
-  __shared__ T xs[kTile * kMaxK];
-  __shared__ T gs[kMaxK * kMaxJ];
-  for (int i = threadIdx.x; i < K * J; i += blockDim.x) gs[i] = T(alpha * G[i]);
-  const T tb = T(beta);
-  const uint64_t ntiles = (n + kTile - 1) / kTile;
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint64_t base = tile * kTile;
-    const int rows = int(min(uint64_t(kTile), n - base));
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < kTile * K; idx += blockDim.x) {
-      int r = idx / K, k = idx - r * K;
-      xs[idx] = r < rows ? X[(base + r) * ldx + xo + k] : T(0);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < rows * J; idx += blockDim.x) {
-      int r = idx / J, j = idx - r * J;
-      T t = T(0);
-      for (int k = 0; k < K; ++k) t = fma(xs[r * K + k], gs[k * J + j], t);
-      T* yp = Y + (base + r) * ldy + yo + j;
-      *yp = (beta == 0.0) ? t : fma(tb, *yp, t);
-    }
-  }
-}
-
-// Residuals of C Ritz candidates: R[:, c] = AB Sc[:, c] - lam[c] B Sc[:, c],
-// with per-CTA partial sums of |R[:, c]|^2.
-template <class T>
-__global__ void __launch_bounds__(kThreads) k_residual(uint64_t n, const T* __restrict__ B, const T* __restrict__ AB,
-                                                       int ld, int K, const double* __restrict__ Sc,
-                                                       const double* __restrict__ lam, int C, T* __restrict__ R,
-                                                       int ldr, double* __restrict__ part, uint64_t rows_per_cta) {
-  __shared__ T bs[kTile * kMaxK];
-  __shared__ T abs_[kTile * kMaxK];
-  __shared__ T ss[kMaxK * kMaxC];
-  __shared__ double red[kThreads];
-  for (int i = threadIdx.x; i < K * C; i += blockDim.x) ss[i] = T(Sc[i]);
-  const int c = threadIdx.x % C, rstep = kThreads / C, r_first = threadIdx.x / C;
-  const bool active = threadIdx.x < rstep * C;
-  const T lc = active ? T(lam[c]) : T(0);
-  double acc = 0.0;
-  const uint64_t r0 = uint64_t(blockIdx.x) * rows_per_cta;
-  const uint64_t r1 = min(n, r0 + rows_per_cta);
-  for (uint64_t base = r0; base < r1; base += kTile) {
-    const int rows = int(min(uint64_t(kTile), r1 - base));
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < kTile * K; idx += blockDim.x) {
-      int r = idx / K, k = idx - r * K;
-      bool ok = r < rows;
-      bs[idx] = ok ? B[(base + r) * ld + k] : T(0);
-      abs_[idx] = ok ? AB[(base + r) * ld + k] : T(0);
-    }
-    __syncthreads();
-    if (active) {
-      T tile = T(0);
-      for (int r = r_first; r < rows; r += rstep) {
-        T a = T(0), b = T(0);
-        for (int k = 0; k < K; ++k) {
-          T s = ss[k * C + c];
-          a = fma(abs_[r * K + k], s, a);
-          b = fma(bs[r * K + k], s, b);
-        }
-        T res = a - lc * b;
-        R[(base + r) * ldr + c] = res;
-        tile = fma(res, res, tile);
-      }
-      acc += double(tile);
-    }
-  }
-  red[threadIdx.x] = active ? acc : 0.0;
-  __syncthreads();
-  if (threadIdx.x < C) {
-    double s = 0.0;
-    for (int t = threadIdx.x; t < rstep * C; t += C) s += red[t];
-    part[uint64_t(blockIdx.x) * C + threadIdx.x] = s;
-  }
-}
-
 // B[:, bo + a] = R[:, sel[a]] / g, g = lam[a] - diag_i, |g| <= 1e-13 -> 1e-13.
+// 1 << sh >= A lanes a row, four rows a thread.
+struct PrecondArgs {
+  int sel[kMaxC];
+  double lam[kMaxC];
+};
 template <class T>
-__global__ void k_precond_copy(uint64_t n, const T* __restrict__ R, int ldr, const int* __restrict__ sel,
-                               const double* __restrict__ lam, int A, const double* __restrict__ diag, T* __restrict__ B,
-                               int ld, int bo) {
-  uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (idx >= n * A) return;
-  uint64_t i = idx / A;
-  int a = int(idx - i * A);
-  // the difference in FP64 (theta and diag agree to many digits near
-  // convergence), the division in the vectors' precision
-  T g = T(lam[a] - diag[i]);
-  if (!(fabs(g) > T(1e-13))) g = T(1e-13);
-  B[i * ld + bo + a] = R[i * ldr + sel[a]] / g;
+__global__ void __launch_bounds__(256) k_precond_copy(uint64_t n, const T* __restrict__ R, int ldr,
+                                                      const __grid_constant__ PrecondArgs pa, int A, int sh,
+                                                      const double* __restrict__ diag, T* __restrict__ B, int ld,
+                                                      int bo) {
+  const int a = threadIdx.x & ((1 << sh) - 1);
+  if (a >= A) return;
+  const int sel = pa.sel[a];
+  const double lam = pa.lam[a];
+  const uint64_t i0 = (blockIdx.x * 1024ull + threadIdx.x) >> sh;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const uint64_t i = i0 + u * (256u >> sh);
+    if (i >= n) return;
+    // the difference in FP64 (theta and diag agree to many digits near
+    // convergence), the division in the vectors' precision
+    T g = T(lam - diag[i]);
+    if (!(fabs(g) > T(1e-13))) g = T(1e-13);
+    B[i * ld + bo + a] = R[i * ldr + sel] / g;
+  }
 }
-
 template <class T>
 __global__ void k_scale_cols(uint64_t n, T* __restrict__ B, int ld, int bo, int J, const double* __restrict__ sc) {
   uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
@@ -841,15 +620,17 @@ __global__ void k_copy_cols(uint64_t n, const T* S, int lds, int so, T* D, int l
 }
 
 // W (n x pad, packed 32/64-byte rows) = B[:, c0:c0+m] padded with zero columns
-__global__ void k_stage_block(uint64_t n, const float* __restrict__ B, int ld, int c0, int m, float* __restrict__ W,
-                              int pad) {
-  uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (idx >= n * pad) return;
-  uint64_t i = idx / pad;
-  int j = int(idx - i * pad);
-  W[idx] = j < m ? B[i * ld + c0 + j] : 0.f;
+__global__ void __launch_bounds__(256) k_stage_block(uint64_t n, const float* __restrict__ B, int ld, int c0, int m,
+                                                     float* __restrict__ W, int sh) {
+  // 1 << sh columns, four rows a thread
+  const int j = threadIdx.x & ((1 << sh) - 1);
+  const uint64_t i0 = (blockIdx.x * 1024ull + threadIdx.x) >> sh;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const uint64_t i = i0 + u * (256u >> sh);
+    if (i < n) W[(i << sh) + j] = j < m ? B[i * ld + c0 + j] : 0.f;
+  }
 }
-
 // W (n x 8 FP32, zero-padded) = columns c0 .. c0+m of the FP64 block B, rounded
 __global__ void k_narrow8(uint64_t n, const double* __restrict__ B, int ld, int c0, int m, float* __restrict__ W) {
   uint64_t idx = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
@@ -904,14 +685,44 @@ struct Engine {
   cudaStream_t s;
   uint64_t n;
   int L;           // leading dimension of B / AB (>= lim, padded)
-  int nparts;      // CTAs of the reduction kernels
   int nsm_ = 1;
   uint64_t xwarps_ = 8, xrows_ = 1;  // warps of the X^T Y kernel and rows per warp
-  uint64_t rows_per_cta;
   DBuf<T> B, AB, R;
   int ldr;
-  DBuf<double> part, small, small2, dlam;
-  DBuf<int> dsel;
+  DBuf<double> part, small2;
+  // Pinned host memory: results of reductions, written by the device, and a
+  // ring of small uploads, which return without a wait
+  struct Pinned {
+    static constexpr size_t kUp = 256 * 1024;
+    double* down = nullptr;  // kMaxLim x 16
+    char* up = nullptr;
+    size_t at = 0;
+    void alloc() {
+      CG_CUDA(cudaMallocHost(&down, sizeof(double) * kMaxLim * 16 + kUp));
+      up = reinterpret_cast<char*>(down + kMaxLim * 16);
+    }
+    ~Pinned() { if (down) cudaFreeHost(down); }
+  } pinned;
+  void upload(double* dst, const double* src, size_t count) {
+    const size_t bytes = sizeof(double) * count;
+    if (bytes > Pinned::kUp) throw Error(CG_ERR_INTERNAL, "upload out of range");
+    if (pinned.at + bytes > Pinned::kUp) wait();
+    std::memcpy(pinned.up + pinned.at, src, bytes);
+    CG_CUDA(cudaMemcpyAsync(dst, pinned.up + pinned.at, bytes, cudaMemcpyHostToDevice, s));
+    pinned.at += bytes;
+  }
+  bool timed_ = false;  // ev0 .. ev1 not yet in spmm_s
+  // for everything enqueued
+  void wait() {
+    CG_CUDA(cudaStreamSynchronize(s));
+    pinned.at = 0;
+    if (timed_) {
+      float ms = 0;
+      CG_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
+      spmm_s += ms * 1e-3;
+      timed_ = false;
+    }
+  }
   DBuf<uint64_t> drows;
   double spmm_s = 0;
   // host wall time per phase (verbose >= 2 prints them)
@@ -941,10 +752,6 @@ struct Engine {
     int nsm = 0;
     CG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h.device));
     nsm_ = nsm;
-    nparts = std::max(1, std::min<int>(nsm * 4, int((n + kTile - 1) / kTile)));
-    rows_per_cta = (n + nparts - 1) / nparts;
-    rows_per_cta = (rows_per_cta + kTile - 1) / kTile * kTile;
-    nparts = int((n + rows_per_cta - 1) / rows_per_cta);
     B.alloc(n * L);
     AB.alloc(n * L);
     // FP32 residual rows padded to 32 bytes (stored 8 columns at a time)
@@ -956,12 +763,9 @@ struct Engine {
     xrows_ = (xrows_ + 3) / 4 * 4;
     xwarps_ = std::max<uint64_t>(8, (n + xrows_ - 1) / xrows_);
     xwarps_ = (xwarps_ + 7) / 8 * 8;
-    part.alloc(std::max<size_t>(std::max<size_t>(size_t(nparts) * kMaxK * kMaxJ, size_t(nsm * 8) * kMaxC),
-                                size_t(xwarps_) * 64 * 16));
-    small.alloc(kMaxLim * kMaxLim);
+    part.alloc(std::max<size_t>(size_t(nsm * 8) * kMaxC, size_t(xwarps_ / 8) * kMaxK * 16));
+    pinned.alloc();
     small2.alloc(kMaxLim * kMaxLim);
-    dlam.alloc(kMaxLim);
-    dsel.alloc(kMaxLim);
     drows.alloc(kMaxLim);
     CG_CUDA(cudaMemsetAsync(B.p, 0, B.bytes(), s));
     CG_CUDA(cudaMemsetAsync(AB.p, 0, AB.bytes(), s));
@@ -973,47 +777,65 @@ struct Engine {
     icv.assign(nume, 0);
   }
   ~Engine() {
+    cudaStreamSynchronize(s);
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
   }
 
-  // G (K x J, row-major, host) = X[:, xo:xo+K]^T Y[:, yo:yo+J]; more than
-  // kMaxK columns of X go through the kernels kMaxK at a time (rows of G)
+  // G (K x J, row-major, host) = X[:, xo:xo+K]^T Y[:, yo:yo+J]; the kernels
+  // take kMaxK columns of X and, but for k_xty_p, 8 of Y at a time
   void xty(const T* X, int xo, int K, const T* Y, int yo, int J, std::vector<double>& G) {
-    if (K > kMaxK && J > 0) {
-      if (K > kMaxLim) throw Error(CG_ERR_INTERNAL, "xty shape out of range");
-      G.assign(size_t(K) * J, 0.0);
-      std::vector<double> Gc;
-      for (int k0 = 0; k0 < K; k0 += kMaxK) {
-        const int kc = std::min(kMaxK, K - k0);
-        xty(X, xo + k0, kc, Y, yo, J, Gc);
-        std::copy(Gc.begin(), Gc.end(), G.begin() + size_t(k0) * J);
+    G.assign(size_t(K) * J, 0.0);
+    if (K == 0 || J == 0) return;
+    if (J > 16 || K > kMaxLim) throw Error(CG_ERR_INTERNAL, "xty shape out of range");
+    for (int k0 = 0; k0 < K; k0 += kMaxK) {
+      const int kc = std::min(kMaxK, K - k0);
+      if constexpr (sizeof(T) == 8) {
+        xty_f64(X, xo + k0, kc, Y, yo, J, pinned.down + size_t(k0) * J);
+      } else {
+        for (int j0 = 0; j0 < J; j0 += 8) {
+          const int jc = std::min(8, J - j0);
+          const unsigned blocks = unsigned(xwarps_ / 8);
+          if (jc <= 4) k_xty_t<4><<<blocks, 256, 0, s>>>(n, X, L, xo + k0, kc, Y, L, yo + j0, jc, part.p, xrows_);
+          else k_xty_t<8><<<blocks, 256, 0, s>>>(n, X, L, xo + k0, kc, Y, L, yo + j0, jc, part.p, xrows_);
+          reduce(int(blocks), kc * jc, pinned.down + size_t(k0) * J + j0, jc, J);
+        }
       }
-      return;
     }
-    if (K == 0 || J == 0) { G.assign(size_t(K) * J, 0.0); return; }
-    if (J > 16 || K > kMaxK) throw Error(CG_ERR_INTERNAL, "xty shape out of range");
+    wait();
+    std::copy(pinned.down, pinned.down + size_t(K) * J, G.begin());
+  }
+  void reduce(int parts, int nout, double* out, int cols, int ldo) {
+    CG_CUDA(cudaGetLastError());
+    count_launch();
+    k_reduce_parts<<<unsigned(nout + 31) / 32, 1024, 0, s>>>(part.p, parts, nout, out, cols, ldo);
+    CG_CUDA(cudaGetLastError());
+    count_launch();
+  }
+  void xty_f64(const double* X, int xo, int K, const double* Y, int yo, int J, double* out) {
     const unsigned blocks = unsigned(xwarps_ / 8);
     // the refinement phase of the mixed solve multiplies in double-float; the
-    // plain FP64 solve (and any product of fewer than 3 columns) stays FP64
-    const bool df = sizeof(T) == 8 && cfg.spmm_prec == CG_PREC_REFINE && J >= 3;
-    if constexpr (sizeof(T) == 8) {
-      if (df && J <= 4) k_xty_df<4><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-      else if (df && J <= 8) k_xty_df<8><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-      else if (J <= 4) k_xty_t<T, 4><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-      else if (J <= 8) k_xty_t<T, 8><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-      else k_xty_w<T, 16><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-    } else if (J <= 4) k_xty_t<T, 4><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-    else if (J <= 8) k_xty_t<T, 8><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-    else k_xty_w<T, 16><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
-    CG_CUDA(cudaGetLastError());
-    count_launch();
-    k_reduce_parts<<<K * J, 128, 0, s>>>(part.p, int(xwarps_), K * J, small.p);
-    CG_CUDA(cudaGetLastError());
-    count_launch();
-    G.resize(size_t(K) * J);
-    CG_CUDA(cudaMemcpyAsync(G.data(), small.p, sizeof(double) * K * J, cudaMemcpyDeviceToHost, s));
-    CG_CUDA(cudaStreamSynchronize(s));
+    // plain FP64 solve (and any product of fewer than 3 or more than 8 columns)
+    // stays FP64
+    if (cfg.spmm_prec == CG_PREC_REFINE && J >= 3 && J <= 8) {
+      if (J <= 4) k_xty_df<4><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
+      else k_xty_df<8><<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo, J, part.p, xrows_);
+      reduce(int(blocks), K * J, out, J, J);
+      return;
+    }
+    const int most = std::min(J, 512 / K);  // columns of Y for at most 16 outputs a lane
+    for (int j0 = 0; j0 < J; j0 += most) {
+      const int jc = std::min(most, J - j0), nt = (K * jc + 31) / 32;
+      const auto go = [&](auto kern) {
+        kern<<<blocks, 256, 0, s>>>(n, X, L, xo, K, Y, L, yo + j0, jc, part.p, xrows_);
+      };
+      if (nt <= 1) go(k_xty_p<1>);
+      else if (nt <= 2) go(k_xty_p<2>);
+      else if (nt <= 4) go(k_xty_p<4>);
+      else if (nt <= 8) go(k_xty_p<8>);
+      else go(k_xty_p<16>);
+      reduce(int(blocks), K * jc, out + j0, jc, J);
+    }
   }
   // Y[:, yo:yo+J] = beta Y + alpha X[:, xo:xo+K] G (G host K x J).  More
   // than kMaxJ outputs (beta 0 only: the thick restart keeping more than 32
@@ -1035,7 +857,6 @@ struct Engine {
       k_copy_cols<T><<<blocks_for(n * uint64_t(J)), 256, 0, s>>>(n, wide_.p, J, 0, Yp, L, yo, J);
       CG_CUDA(cudaGetLastError());
       count_launch();
-      CG_CUDA(cudaStreamSynchronize(s));
       return;
     }
     gemm_ld(Xp, xo, K, G, Yp, L, yo, J, alpha, beta);
@@ -1047,7 +868,7 @@ struct Engine {
     if (K < 0 || K > kMaxLim || J < 0 || J > kMaxJ) throw Error(CG_ERR_INTERNAL, "gemm shape out of range");
     const bool wide = K > kMaxK;
     if (K == 0 || J == 0) return;
-    CG_CUDA(cudaMemcpyAsync(small2.p, G.data(), sizeof(double) * K * J, cudaMemcpyHostToDevice, s));
+    upload(small2.p, G.data(), size_t(K) * J);
     const bool vx = reinterpret_cast<uintptr_t>(Xp + xo) % 32 == 0 && L % 8 == 0;
     const bool vy = reinterpret_cast<uintptr_t>(Yp + yo) % 32 == 0 && ldy % 8 == 0 && J % 8 == 0;
     unsigned grid = unsigned(std::min<uint64_t>((n + 255) / 256, uint64_t(nsm_) * 8));
@@ -1063,7 +884,6 @@ struct Engine {
 #undef CG_GEMM_DF
         CG_CUDA(cudaGetLastError());
         count_launch();
-        CG_CUDA(cudaStreamSynchronize(s));
         return;
       }
     }
@@ -1093,7 +913,6 @@ struct Engine {
 #undef CG_GEMM_R
     CG_CUDA(cudaGetLastError());
     count_launch();
-    CG_CUDA(cudaStreamSynchronize(s));  // G's staging buffer is reused by the next call
   }
   DBuf<float> stage;  // FP32 engine: aligned SpMM input block (n x 16)
   // Refinement phase: once the starting vectors' products are in AB (double-
@@ -1127,6 +946,7 @@ struct Engine {
     }
   }
   void spmm(int c0, int m) {
+    if (timed_) wait();
     CG_CUDA(cudaEventRecord(ev0, s));
     if (fp32_corr_) {
       spmm_narrow(c0, m);
@@ -1161,8 +981,8 @@ struct Engine {
         const int most = H.use_fact() ? 8 : 16;
         for (int c = 0; c < m; c += most) {
           const int mc = std::min(most, m - c), pad = mc <= 8 ? 8 : 16;
-          k_stage_block<<<blocks_for(n * pad), 256, 0, s>>>(n, reinterpret_cast<const float*>(B.p), L, c0 + c, mc,
-                                                              stage.p, pad);
+          k_stage_block<<<unsigned((n * pad + 1023) / 1024), 256, 0, s>>>(n, reinterpret_cast<const float*>(B.p), L,
+                                                                          c0 + c, mc, stage.p, mc <= 8 ? 3 : 4);
           CG_CUDA(cudaGetLastError());
           count_launch();
           spmm_f32_padded(H, stage.p, pad, reinterpret_cast<float*>(AB.p) + c0 + c, L, mc, s);
@@ -1178,10 +998,7 @@ struct Engine {
       spmm_launch(H, cfg.spmm_prec, B.p + c0, L, AB.p + c0, L, m, s);
     }
     CG_CUDA(cudaEventRecord(ev1, s));
-    CG_CUDA(cudaEventSynchronize(ev1));
-    float ms = 0;
-    CG_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
-    spmm_s += ms * 1e-3;
+    timed_ = true;
   }
   // new columns of S from AB[:, c0:c0+m] (Add_Vectors_To_AB_S, fsdavidson.cxx:161-211)
   void add_ab_s(int c0, int m, int64_t& nmv) {
@@ -1234,8 +1051,9 @@ struct Engine {
       lam[c] = eigs[st[c]];
       for (int k = 0; k < kpass; ++k) Sc[size_t(k) * C + c] = svec(st[c], k);
     }
-    CG_CUDA(cudaMemcpyAsync(small2.p, Sc.data(), sizeof(double) * Sc.size(), cudaMemcpyHostToDevice, s));
-    CG_CUDA(cudaMemcpyAsync(dlam.p, lam.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
+    Sc.insert(Sc.end(), lam.begin(), lam.end());
+    upload(small2.p, Sc.data(), Sc.size());
+    const double* dlam = small2.p + size_t(kpass) * C;
     const unsigned rgrid = unsigned(std::min<uint64_t>((n + 255) / 256, uint64_t(nsm_) * 8));
     const bool vec = L % 8 == 0 && reinterpret_cast<uintptr_t>(B.p) % 32 == 0 &&
                      reinterpret_cast<uintptr_t>(AB.p) % 32 == 0;
@@ -1245,45 +1063,46 @@ struct Engine {
       if (cfg.spmm_prec == CG_PREC_REFINE) {
         const bool v4 = L % 4 == 0 && reinterpret_cast<uintptr_t>(B.p) % 32 == 0 &&
                         reinterpret_cast<uintptr_t>(AB.p) % 32 == 0;
-#define CG_RESID_DF(CM, KM) k_resid_df<CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam.p, C, R.p, ldr, part.p, v4)
+#define CG_RESID_DF(CM, KM) k_resid_df<CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam, C, R.p, ldr, part.p, v4)
         if (C <= 8) { if (kpass > kMaxK) CG_RESID_DF(8, kMaxLim); else CG_RESID_DF(8, kMaxK); }
+        else if (C <= 12) { if (kpass > kMaxK) CG_RESID_DF(12, kMaxLim); else CG_RESID_DF(12, kMaxK); }
         else { if (kpass > kMaxK) CG_RESID_DF(16, kMaxLim); else CG_RESID_DF(16, kMaxK); }
 #undef CG_RESID_DF
         done = true;
       }
     }
     if (!done) {
-#define CG_RESID_V(CM, KM) k_resid_v<T, CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam.p, C, R.p, ldr, part.p, vec, vec_r)
+#define CG_RESID_V(CM, KM) k_resid_v<T, CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam, C, R.p, ldr, part.p, vec, vec_r)
       if (C <= 8) { if (kpass > kMaxK) CG_RESID_V(8, kMaxLim); else CG_RESID_V(8, kMaxK); }
+      else if (C <= 12) { if (kpass > kMaxK) CG_RESID_V(12, kMaxLim); else CG_RESID_V(12, kMaxK); }
       else { if (kpass > kMaxK) CG_RESID_V(16, kMaxLim); else CG_RESID_V(16, kMaxK); }
 #undef CG_RESID_V
     }
-    CG_CUDA(cudaGetLastError());
-    count_launch();
-    k_reduce_parts<<<C, 128, 0, s>>>(part.p, int(rgrid), C, small.p);
-    CG_CUDA(cudaGetLastError());
-    count_launch();
-    std::vector<double> nr(C);
-    CG_CUDA(cudaMemcpyAsync(nr.data(), small.p, sizeof(double) * C, cudaMemcpyDeviceToHost, s));
-    CG_CUDA(cudaStreamSynchronize(s));
+    reduce(int(rgrid), C, pinned.down, C, C);
+    wait();
+    std::vector<double> nr(pinned.down, pinned.down + C);
     for (auto& x : nr) x = std::sqrt(std::max(x, 0.0));
     return nr;
   }
   void precond_copy(const std::vector<int>& sel_r, const std::vector<double>& lam, int bo) {
     int A = int(sel_r.size());
     if (!A) return;
-    CG_CUDA(cudaMemcpyAsync(dsel.p, sel_r.data(), sizeof(int) * A, cudaMemcpyHostToDevice, s));
-    CG_CUDA(cudaMemcpyAsync(dlam.p, lam.data(), sizeof(double) * A, cudaMemcpyHostToDevice, s));
-    k_precond_copy<T><<<blocks_for(n * A), 256, 0, s>>>(n, R.p, ldr, dsel.p, dlam.p, A, H.diag.p, B.p, L, bo);
+    if (A > kMaxC) throw Error(CG_ERR_INTERNAL, "preconditioner shape out of range");
+    PrecondArgs pa = {};
+    std::copy(sel_r.begin(), sel_r.end(), pa.sel);
+    std::copy(lam.begin(), lam.begin() + A, pa.lam);
+    int sh = 0;
+    while (1 << sh < A) ++sh;
+    const unsigned grid = unsigned(((n << sh) + 1023) / 1024);
+    k_precond_copy<T><<<grid, 256, 0, s>>>(n, R.p, ldr, pa, A, sh, H.diag.p, B.p, L, bo);
     CG_CUDA(cudaGetLastError());
     count_launch();
   }
   void scale_col(int c, double f) {
-    CG_CUDA(cudaMemcpyAsync(small2.p, &f, sizeof(double), cudaMemcpyHostToDevice, s));
+    upload(small2.p, &f, 1);
     k_scale_cols<T><<<blocks_for(n), 256, 0, s>>>(n, B.p, L, c, 1, small2.p);
     CG_CUDA(cudaGetLastError());
     count_launch();
-    CG_CUDA(cudaStreamSynchronize(s));
   }
   void copy_col(int from, int to) {
     k_copy_cols<T><<<blocks_for(n), 256, 0, s>>>(n, B.p, L, from, B.p, L, to, 1);
@@ -1343,11 +1162,10 @@ struct Engine {
   }
   void gram(int basis_dim, int m, std::vector<double>& M) { xty(B.p, basis_dim, m, B.p, basis_dim, m, M); }
   void scale_block(int basis_dim, int m, const std::vector<double>& f) {
-    CG_CUDA(cudaMemcpyAsync(small2.p, f.data(), sizeof(double) * m, cudaMemcpyHostToDevice, s));
+    upload(small2.p, f.data(), size_t(m));
     k_scale_cols<T><<<blocks_for(n * m), 256, 0, s>>>(n, B.p, L, basis_dim, m, small2.p);
     CG_CUDA(cudaGetLastError());
     count_launch();
-    CG_CUDA(cudaStreamSynchronize(s));
   }
   // Block Gram-Schmidt with Pythagorean inner products, twice (BCGS-PIP2):
   // one X^T Y over [basis | block] gives the projections G = X^T Y and the
@@ -1639,6 +1457,7 @@ struct Engine {
     out.iterations = nloops;
     out.matvecs = nmv;
     out.ierr = done ? 0 : (ierr_stall ? 1024 : 2048);
+    wait();
     out.spmm_seconds = spmm_s;
     out.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (cfg.verbose >= 2)
@@ -1823,6 +1642,7 @@ struct Engine {
     out.iterations = nloops;
     out.matvecs = nmv;
     out.ierr = ierr;
+    wait();
     out.spmm_seconds = spmm_s;
     out.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return out;
