@@ -25,6 +25,7 @@
 #include <cstdio>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 
 #include "davidson.h"
 #include "dfloat.h"
@@ -412,6 +413,17 @@ __device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
                : "memory");
 }
 
+// Weights of the thread-per-row kernels: FP32 as a kernel parameter (no upload),
+// FP64 in device memory, staged in shared memory.
+template <class T, int N>
+struct Weights {
+  T v[N];
+};
+template <int N>
+struct Weights<double, N> {
+  const double* p;
+};
+
 // R[:, c] = AB s_c - lam_c B s_c for C <= CMAX candidates (for 10, rounding up to
 // 12 instead of 16: 2e6 rows of 96 columns 0.45 -> 0.35 ms, in double-float 1.04
 // -> 0.67), one thread per row with the
@@ -420,18 +432,28 @@ __device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
 // thread's rows, FP64 across threads, fixed order).
 template <class T, int CMAX, int KM>
 __global__ void __launch_bounds__(256) k_resid_v(uint64_t n, const T* __restrict__ B, const T* __restrict__ AB,
-                                                 int ld, int K, const double* __restrict__ Sc,
-                                                 const double* __restrict__ lam, int C, T* __restrict__ R, int ldr,
-                                                 double* __restrict__ part, bool vec, bool vec_r) {
-  __shared__ __align__(16) T ss[KM * CMAX];
-  __shared__ T ls[CMAX];
+                                                 int ld, int K,
+                                                 const __grid_constant__ Weights<T, (KM + 1) * CMAX> wt, int C,
+                                                 T* __restrict__ R, int ldr, double* __restrict__ part, bool vec,
+                                                 bool vec_r) {
   __shared__ double red[8][CMAX];
-  for (int i = threadIdx.x; i < KM * CMAX; i += blockDim.x) {
-    const int k = i / CMAX, c = i % CMAX;
-    ss[i] = (k < K && c < C) ? T(Sc[k * C + c]) : T(0);
+  // lam and s, CMAX a row.  FP32 through the constant bank: in shared memory their
+  // reads took a third of the L1 pipe, which bounds the kernel with the loads of
+  // 32 rows at a time (2e6 rows of 96 columns, 10 candidates: 0.35 -> 0.28 ms).
+  const T *ls, *ss;
+  if constexpr (sizeof(T) == 4) {
+    ls = wt.v;
+    ss = wt.v + CMAX;
+  } else {
+    __shared__ __align__(16) T ws[(KM + 1) * CMAX];
+    for (int i = threadIdx.x; i < (KM + 1) * CMAX; i += blockDim.x) {
+      const int k = i / CMAX, c = i % CMAX;
+      ws[i] = (k <= K && c < C) ? wt.p[k * C + c] : 0.0;
+    }
+    __syncthreads();
+    ls = ws;
+    ss = ws + CMAX;
   }
-  for (int i = threadIdx.x; i < CMAX; i += blockDim.x) ls[i] = i < C ? T(lam[i]) : T(0);
-  __syncthreads();
   T nrm[CMAX];
 #pragma unroll
   for (int c = 0; c < CMAX; ++c) nrm[c] = T(0);
@@ -501,17 +523,23 @@ __global__ void __launch_bounds__(256) k_resid_v(uint64_t n, const T* __restrict
 }
 
 // Y[:, yo:yo+J] = beta Y + alpha X[:, xo:xo+K] G, one thread per row, all J
-// outputs of the row in registers, G (alpha folded in) in shared memory read
-// as broadcast; FP32 X rows read 8 values (32 bytes) at a time when aligned.  A row is
-// read completely before it is written, so X and Y may alias.
+// outputs of the row in registers, alpha folded into G; FP32 X rows read 8 values
+// (32 bytes) at a time when aligned.  A row is read completely before it is
+// written, so X and Y may alias.
 template <class T, int JMAX, int KM>
 __global__ void __launch_bounds__(256) k_gemm_r(uint64_t n, const T* X, int ldx, int xo, int K,
-                                                const double* __restrict__ G, T* Y, int ldy, int yo, int J,
-                                                double alpha, double beta, bool vec_x, bool vec_y) {
+                                                const __grid_constant__ Weights<T, KM * JMAX> G, T* Y, int ldy,
+                                                int yo, int J, double beta, bool vec_x, bool vec_y) {
+  // in shared memory: through the constant bank, one multiply-add a read and row,
+  // 2e6 rows of 96 columns x 8 took 0.29 ms instead of 0.19
   __shared__ __align__(16) T gs[KM * JMAX];
-  for (int i = threadIdx.x; i < KM * JMAX; i += blockDim.x) {
-    const int k = i / JMAX, j = i % JMAX;
-    gs[i] = (k < K && j < J) ? T(alpha * G[k * J + j]) : T(0);
+  if constexpr (sizeof(T) == 4) {
+    for (int i = threadIdx.x; i < K * JMAX; i += blockDim.x) gs[i] = G.v[i];
+  } else {
+    for (int i = threadIdx.x; i < K * JMAX; i += blockDim.x) {
+      const int k = i / JMAX, j = i % JMAX;
+      gs[i] = j < J ? G.p[k * J + j] : 0.0;
+    }
   }
   __syncthreads();
   const T tb = T(beta);
@@ -868,12 +896,12 @@ struct Engine {
     if (K < 0 || K > kMaxLim || J < 0 || J > kMaxJ) throw Error(CG_ERR_INTERNAL, "gemm shape out of range");
     const bool wide = K > kMaxK;
     if (K == 0 || J == 0) return;
-    upload(small2.p, G.data(), size_t(K) * J);
     const bool vx = reinterpret_cast<uintptr_t>(Xp + xo) % 32 == 0 && L % 8 == 0;
     const bool vy = reinterpret_cast<uintptr_t>(Yp + yo) % 32 == 0 && ldy % 8 == 0 && J % 8 == 0;
     unsigned grid = unsigned(std::min<uint64_t>((n + 255) / 256, uint64_t(nsm_) * 8));
     if constexpr (sizeof(T) == 8) {
       if (J <= 32 && J >= 3 && cfg.spmm_prec == CG_PREC_REFINE) {
+        upload(small2.p, G.data(), size_t(K) * J);
         const double* Xd = reinterpret_cast<const double*>(Xp);
         double* Yd = reinterpret_cast<double*>(Yp);
         const bool v4 = reinterpret_cast<uintptr_t>(Xp + xo) % 32 == 0 && L % 4 == 0;
@@ -887,30 +915,36 @@ struct Engine {
         return;
       }
     }
-    // one wave of resident CTAs (the grid-stride loop gives each thread whole
-    // rows, so the grid changes no result)
-    const int jc = (J <= 4 ? 0 : J <= 8 ? 1 : J <= 16 ? 2 : 3) + (wide ? 4 : 0);
-    if (!gemm_occ_[jc]) {
-      int per_sm = 0;
-      switch (jc) {
-        case 0: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 4, kMaxK>, 256, 0)); break;
-        case 1: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 8, kMaxK>, 256, 0)); break;
-        case 2: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 16, kMaxK>, 256, 0)); break;
-        case 3: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 32, kMaxK>, 256, 0)); break;
-        case 4: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 4, kMaxLim>, 256, 0)); break;
-        case 5: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 8, kMaxLim>, 256, 0)); break;
-        case 6: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 16, kMaxLim>, 256, 0)); break;
-        default: CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, 32, kMaxLim>, 256, 0)); break;
+    const auto go = [&](auto jm, auto km, int slot) {
+      constexpr int JM = decltype(jm)::value, KM = decltype(km)::value;
+      Weights<T, KM * JM> w;
+      if constexpr (sizeof(T) == 4) {
+        for (int k = 0; k < K; ++k)
+          for (int j = 0; j < JM; ++j) w.v[k * JM + j] = j < J ? T(alpha * G[size_t(k) * J + j]) : T(0);
+      } else {
+        std::vector<double> ag(G);
+        for (double& g : ag) g *= alpha;
+        upload(small2.p, ag.data(), size_t(K) * J);
+        w.p = small2.p;
       }
-      gemm_occ_[jc] = std::max(per_sm, 1);
-    }
-    grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, uint64_t(nsm_) * gemm_occ_[jc])));
-#define CG_GEMM_R(JM, KM) k_gemm_r<T, JM, KM><<<grid, 256, 0, s>>>(n, Xp, L, xo, K, small2.p, Yp, ldy, yo, J, alpha, beta, vx, vy)
-    if (J <= 4) { if (wide) CG_GEMM_R(4, kMaxLim); else CG_GEMM_R(4, kMaxK); }
-    else if (J <= 8) { if (wide) CG_GEMM_R(8, kMaxLim); else CG_GEMM_R(8, kMaxK); }
-    else if (J <= 16) { if (wide) CG_GEMM_R(16, kMaxLim); else CG_GEMM_R(16, kMaxK); }
-    else { if (wide) CG_GEMM_R(32, kMaxLim); else CG_GEMM_R(32, kMaxK); }
-#undef CG_GEMM_R
+      // one wave of resident CTAs (the grid-stride loop gives each thread whole
+      // rows, so the grid changes no result)
+      if (!gemm_occ_[slot]) {
+        int per_sm = 0;
+        CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gemm_r<T, JM, KM>, 256, 0));
+        gemm_occ_[slot] = std::max(per_sm, 1);
+      }
+      grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, uint64_t(nsm_) * gemm_occ_[slot])));
+      k_gemm_r<T, JM, KM><<<grid, 256, 0, s>>>(n, Xp, L, xo, K, w, Yp, ldy, yo, J, beta, vx, vy);
+    };
+    const auto pick = [&](auto km, int first) {
+      if (J <= 4) go(std::integral_constant<int, 4>{}, km, first);
+      else if (J <= 8) go(std::integral_constant<int, 8>{}, km, first + 1);
+      else if (J <= 16) go(std::integral_constant<int, 16>{}, km, first + 2);
+      else go(std::integral_constant<int, 32>{}, km, first + 3);
+    };
+    if (wide) pick(std::integral_constant<int, kMaxLim>{}, 4);
+    else pick(std::integral_constant<int, kMaxK>{}, 0);
     CG_CUDA(cudaGetLastError());
     count_launch();
   }
@@ -1051,19 +1085,18 @@ struct Engine {
       lam[c] = eigs[st[c]];
       for (int k = 0; k < kpass; ++k) Sc[size_t(k) * C + c] = svec(st[c], k);
     }
-    Sc.insert(Sc.end(), lam.begin(), lam.end());
-    upload(small2.p, Sc.data(), Sc.size());
-    const double* dlam = small2.p + size_t(kpass) * C;
+    Sc.insert(Sc.begin(), lam.begin(), lam.end());  // row 0: lam
     const unsigned rgrid = unsigned(std::min<uint64_t>((n + 255) / 256, uint64_t(nsm_) * 8));
     const bool vec = L % 8 == 0 && reinterpret_cast<uintptr_t>(B.p) % 32 == 0 &&
                      reinterpret_cast<uintptr_t>(AB.p) % 32 == 0;
     const bool vec_r = ldr % 8 == 0 && (C + 7) / 8 * 8 <= ldr && reinterpret_cast<uintptr_t>(R.p) % 32 == 0;
     bool done = false;
     if constexpr (sizeof(T) == 8) {
+      upload(small2.p, Sc.data(), Sc.size());
       if (cfg.spmm_prec == CG_PREC_REFINE) {
         const bool v4 = L % 4 == 0 && reinterpret_cast<uintptr_t>(B.p) % 32 == 0 &&
                         reinterpret_cast<uintptr_t>(AB.p) % 32 == 0;
-#define CG_RESID_DF(CM, KM) k_resid_df<CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam, C, R.p, ldr, part.p, v4)
+#define CG_RESID_DF(CM, KM) k_resid_df<CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p + C, small2.p, C, R.p, ldr, part.p, v4)
         if (C <= 8) { if (kpass > kMaxK) CG_RESID_DF(8, kMaxLim); else CG_RESID_DF(8, kMaxK); }
         else if (C <= 12) { if (kpass > kMaxK) CG_RESID_DF(12, kMaxLim); else CG_RESID_DF(12, kMaxK); }
         else { if (kpass > kMaxK) CG_RESID_DF(16, kMaxLim); else CG_RESID_DF(16, kMaxK); }
@@ -1072,11 +1105,24 @@ struct Engine {
       }
     }
     if (!done) {
-#define CG_RESID_V(CM, KM) k_resid_v<T, CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, small2.p, dlam, C, R.p, ldr, part.p, vec, vec_r)
-      if (C <= 8) { if (kpass > kMaxK) CG_RESID_V(8, kMaxLim); else CG_RESID_V(8, kMaxK); }
-      else if (C <= 12) { if (kpass > kMaxK) CG_RESID_V(12, kMaxLim); else CG_RESID_V(12, kMaxK); }
-      else { if (kpass > kMaxK) CG_RESID_V(16, kMaxLim); else CG_RESID_V(16, kMaxK); }
-#undef CG_RESID_V
+      const auto go = [&](auto cm, auto km) {
+        constexpr int CM = decltype(cm)::value, KM = decltype(km)::value;
+        Weights<T, (KM + 1) * CM> w;
+        if constexpr (sizeof(T) == 4) {
+          for (int k = 0; k <= kpass; ++k)
+            for (int c = 0; c < CM; ++c) w.v[k * CM + c] = c < C ? T(Sc[size_t(k) * C + c]) : T(0);
+        } else {
+          w.p = small2.p;
+        }
+        k_resid_v<T, CM, KM><<<rgrid, 256, 0, s>>>(n, B.p, AB.p, L, kpass, w, C, R.p, ldr, part.p, vec, vec_r);
+      };
+      const auto pick = [&](auto km) {
+        if (C <= 8) go(std::integral_constant<int, 8>{}, km);
+        else if (C <= 12) go(std::integral_constant<int, 12>{}, km);
+        else go(std::integral_constant<int, 16>{}, km);
+      };
+      if (kpass > kMaxK) pick(std::integral_constant<int, kMaxLim>{});
+      else pick(std::integral_constant<int, kMaxK>{});
     }
     reduce(int(rgrid), C, pinned.down, C, C);
     wait();
