@@ -515,8 +515,13 @@ __global__ void __launch_bounds__(256) k_bxty(const BatchChunk* __restrict__ til
     }
 #pragma unroll
     for (int j = 0; j < kMaxB; ++j) {
-      d0[j] += double(sh0[j]) + double(sl0[j]);
-      if constexpr (HI) d1[j] += double(sh1[j]) + double(sl1[j]);
+      if constexpr (DF) {
+        d0[j] += df_widen(sh0[j]) + df_widen(sl0[j]);
+        if constexpr (HI) d1[j] += df_widen(sh1[j]) + df_widen(sl1[j]);
+      } else {
+        d0[j] += df_widen(sh0[j]);
+        if constexpr (HI) d1[j] += df_widen(sh1[j]);
+      }
     }
   }
 #pragma unroll
@@ -614,7 +619,7 @@ __global__ void __launch_bounds__(256) k_bgemm(const BatchChunk* __restrict__ ti
 #pragma unroll
     for (int j = 0; j < MJ; ++j)
       if (j < J) {
-        const T v = DF ? T(double(ah[j]) + double(al[j])) : T(ah[j]);
+        const T v = DF ? T(df_widen(ah[j]) + df_widen(al[j])) : T(ah[j]);
         yr[j] = beta == 0.0 ? v : T(beta) * yr[j] + v;
       }
   }
@@ -671,7 +676,7 @@ __global__ void __launch_bounds__(256) k_bresid(const BatchChunk* __restrict__ t
     for (int j = 0; j < kMaxB; ++j)
       if (j < b) {
         if constexpr (DF)
-          R[size_t(r) * ldr + j] = T((double(ah[j]) + double(al[j])) - th[j] * (double(bh[j]) + double(bl[j])));
+          R[size_t(r) * ldr + j] = T((df_widen(ah[j]) + df_widen(al[j])) - th[j] * (df_widen(bh[j]) + df_widen(bl[j])));
         else
           R[size_t(r) * ldr + j] = T(ah[j] - float(th[j]) * bh[j]);
       }

@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(256, 4) k_xty_df(uint64_t n, const double* __r
     }
 #pragma unroll
     for (int j = 0; j < JMAX; ++j) {
-      dsh[wl][j][lane] += double(c0h[j]) + double(c0l[j]);
-      dsh[wl][JMAX + j][lane] += double(c1h[j]) + double(c1l[j]);
+      dsh[wl][j][lane] += df_widen(c0h[j]) + df_widen(c0l[j]);
+      dsh[wl][JMAX + j][lane] += df_widen(c1h[j]) + df_widen(c1l[j]);
     }
   }
   store_part<JMAX>(dsh, K, J, part);
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) k_resid_df(uint64_t n, const double* __re
 #pragma unroll
     for (int c = 0; c < CMAX; ++c)
       if (c < C) {
-        const double res = (double(ah[c]) + double(al[c])) - ls[c] * (double(bh[c]) + double(bl[c]));
+        const double res = (df_widen(ah[c]) + df_widen(al[c])) - ls[c] * (df_widen(bh[c]) + df_widen(bl[c]));
         R[r * ldr + c] = res;
         nrm[c] += res * res;
       }
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256) k_gemm_df(uint64_t n, const double* X, in
 #pragma unroll
     for (int j = 0; j < JMAX; ++j)
       if (j < J) {
-        const double v = double(ah[j]) + double(al[j]);
+        const double v = df_widen(ah[j]) + df_widen(al[j]);
         yr[j] = beta == 0.0 ? v : fma(beta, yr[j], v);
       }
   }
@@ -385,8 +385,8 @@ __global__ void __launch_bounds__(256, 4) k_xty_t(uint64_t n, const float* __res
     }
 #pragma unroll
     for (int j = 0; j < JMAX; ++j) {
-      dsh[wl][j][lane] += double(c0v[j]);
-      dsh[wl][JMAX + j][lane] += double(c1v[j]);
+      dsh[wl][j][lane] += df_widen(c0v[j]);
+      dsh[wl][JMAX + j][lane] += df_widen(c1v[j]);
     }
   }
   store_part<JMAX>(dsh, K, J, part);
