@@ -169,13 +169,14 @@ def run_spmm_only(args):
         else:
             tune = H.autotune(args.nvec)
         if args.format:
-            H.set_format(cg.CG_FORMAT_TILED if args.format == "tiled" else cg.CG_FORMAT_ROWS)
+            H.set_format({"tiled": cg.CG_FORMAT_TILED, "rows": cg.CG_FORMAT_ROWS,
+                          "factored": cg.CG_FORMAT_FACTORED}[args.format])
             tune["format_fixed"] = args.format
         if args.tiled_shape:
             r, st = (int(v) for v in args.tiled_shape.split("x"))
             H.set_tiled_shape(r, st)
             tune["tiled_shape"] = args.tiled_shape
-        spmm_s, alg = spmm_roofline(cg, H, args.nvec, reps=args.steps, warm=args.warmup)
+        spmm_s, alg = spmm_roofline(cg, H, args.nvec, reps=args.steps, warm=args.warmup, slots=pair_slots(prob))
     else:
         spmm_s, alg = spmm_roofline(cg, H, args.nvec, reps=args.steps, warm=args.warmup, fp64=True)
     peak, kind = measured_peaks()
@@ -211,10 +212,17 @@ def run_batched_only(args):
                       "states_converged": int(nconv.sum()), "max_resid": float(np.nanmax(res))}))
 
 
-def spmm_roofline(cg, h, b: int, reps: int = 20, warm: int = 3, fp64: bool = False):
+def pair_slots(prob) -> int:
+    """Pairs of particles of a determinant: partial sums a row of the factored product."""
+    kn, kp = int(prob.info.nv), int(prob.info.zv)
+    return kn * kp + kn * (kn - 1) // 2 + kp * (kp - 1) // 2
+
+
+def spmm_roofline(cg, h, b: int, reps: int = 20, warm: int = 3, fp64: bool = False, slots: int = 0):
     """Average device time of one SpMM launch (b vectors) from CUDA events on the
     library's stream, and its algorithmic bytes per launch: stored entries x
-    (value + 4-byte column) + row pointers + the input and output vectors."""
+    (value + 4-byte column) + row pointers + the input and output vectors; the
+    factored product's are its partial sums (slots a row), written and read."""
     import torch
     n = h.n
     esz = 8 if fp64 else 4
@@ -236,8 +244,14 @@ def spmm_roofline(cg, h, b: int, reps: int = 20, warm: int = 3, fp64: bool = Fal
     e1.synchronize()
     ms = e0.elapsed_time(e1) / reps
     nnz = int(h.info.nnz_full)
-    fi = None if fp64 else h.format_info()
-    if fi and fi["format"] == cg.CG_FORMAT_TILED and b <= 8:
+    fmt = cg.CG_FORMAT_ROWS if fp64 else h.format_in_use()
+    fi = h.format_info() if fmt == cg.CG_FORMAT_TILED else None
+    if fmt == cg.CG_FORMAT_FACTORED:
+        # 8 vectors a pass: x gathered from L2 (read once from memory), one
+        # 32-byte partial row a slot written and read, y written
+        alg = (b + 7) // 8 * n * 32 * (1 + 2 * slots) + n * b * 4
+        kernel = "k_fact32+k_pair32+k_fsum"
+    elif fi and b <= 8:
         # tiled: 16-bit column + FP32 value per stored entry (padding excluded;
         # a scaled-identity tile reads one value), x read once (8-wide rows),
         # y written, unit descriptors and run offsets
@@ -321,20 +335,21 @@ def run_ours(args):
     e2e = statistics.median(e2e_times)
 
     # SpMM roofline (FP32 mixed kernel, block of 10 vectors)
-    spmm_s, alg_bytes = spmm_roofline(cg, H, MIXED["block"])
+    spmm_s, alg_bytes = spmm_roofline(cg, H, MIXED["block"], slots=pair_slots(prob))
     # the product's dominant traffic is one 32-byte vector gather per stored
     # entry; its ceiling is the device's random-gather rate over a table the
     # size of the vector block (L2 resident)
     gathers = int(H.info.nnz_full)
     g_peak = cg.gather_ceiling(int(H.n), 1)
     kernel_name = spmm_roofline.kernel
-    fmt_info = H.format_info()
+    fmt = H.format_in_use()
+    fmt_info = H.format_info() if fmt == cg.CG_FORMAT_TILED else {"format": fmt}
     rows_ms = None
-    if fmt_info["format"] == cg.CG_FORMAT_TILED:
+    if fmt != cg.CG_FORMAT_ROWS:
         # the row-wise kernel on the same matrix, for comparison (and its gather rate)
         H.set_format(cg.CG_FORMAT_ROWS)
         rows_s, _ = spmm_roofline(cg, H, MIXED["block"])
-        H.set_format(cg.CG_FORMAT_TILED)
+        H.set_format(fmt)
         rows_ms = rows_s * 1e3
         spmm_roofline.kernel = kernel_name
     peak, peak_kind = measured_peaks()
@@ -754,7 +769,8 @@ def main():
     ap.add_argument("--nvec", type=int, default=10)
     ap.add_argument("--precision", default="fp32", choices=["fp32", "fp64"])
     ap.add_argument("--tuning", default=None, help="fixed launch shape WARPSxCTAS for --mode spmm")
-    ap.add_argument("--format", default=None, choices=["rows", "tiled"], help="fixed SpMM storage for --mode spmm")
+    ap.add_argument("--format", default=None, choices=["rows", "tiled", "factored"],
+                    help="fixed SpMM storage for --mode spmm")
     ap.add_argument("--tiled-shape", default=None, help="tiled product shape SLICESxSTAGES for --mode spmm")
     args = ap.parse_args()
     if args.mode == "spmm":
