@@ -593,13 +593,19 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
   const uint64_t n = h.n;
   // n packed rows of 32 bytes in every precision, kept with the handle
   const DBuf<unsigned char>& pack = h.virt->pack;
+  // Rows that are packed already are taken as they are, unless y overlaps them:
+  // a CTA of the product gathers rows of x whose y another CTA writes.
+  const auto direct = [&](int mc, int vb, size_t elem) {
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), y0 = reinterpret_cast<uintptr_t>(y);
+    const uintptr_t x1 = x0 + n * ldx * elem, y1 = y0 + n * ldy * elem;
+    return mc == vb && ldx == vb && x0 % 32 == 0 && (y1 <= x0 || x1 <= y0);
+  };
   if (precision == CG_PREC_FP32) {
     float* w = reinterpret_cast<float*>(pack.p);
     const float* xf = static_cast<const float*>(x);
     for (int c0 = 0; c0 < m; c0 += kVirtualVB32) {
       const int mc = std::min(kVirtualVB32, m - c0);
-      // rows that are packed already are taken as they are
-      const bool packed = mc == kVirtualVB32 && ldx == kVirtualVB32 && reinterpret_cast<uintptr_t>(x) % 32 == 0;
+      const bool packed = direct(mc, kVirtualVB32, sizeof(float));
       if (!packed) virtual_pack_f32(n, xf, ldx, c0, mc, w, s);
       virtual_product_f32(h, packed ? xf : w, static_cast<float*>(y) + c0, ldy, mc, s);
     }
@@ -615,7 +621,7 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
     const double* xd = static_cast<const double*>(x);
     for (int c0 = 0; c0 < m; c0 += kVirtualVB64) {
       const int mc = std::min(kVirtualVB64, m - c0);
-      const bool packed = mc == kVirtualVB64 && ldx == kVirtualVB64 && reinterpret_cast<uintptr_t>(x) % 32 == 0;
+      const bool packed = direct(mc, kVirtualVB64, sizeof(double));
       if (!packed) virtual_pack_f64(n, xd, ldx, c0, mc, w, s);
       virtual_product_f64(h, packed ? xd : w, static_cast<double*>(y) + c0, ldy, mc, s);
     }

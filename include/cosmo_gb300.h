@@ -200,7 +200,9 @@ void* cg_hamiltonian_stream(const cg_hamiltonian* h);
 cg_status cg_spmm(const cg_hamiltonian* h, const double* x, double* y, int32_t m, int32_t precision);
 /* Device-resident product on the handle's stream: x and y are row-interleaved
  * n x ld arrays (element (i, k) at i*ld + k) of float (CG_PREC_FP32) or double
- * (CG_PREC_FP64, CG_PREC_REFINE); columns [0, m) are used.  Asynchronous. */
+ * (CG_PREC_FP64, CG_PREC_REFINE); columns [0, m) are used.  Asynchronous.
+ * An on-the-fly Hamiltonian takes y = x (with ldy = ldx); for a stored one x
+ * and y must not overlap. */
 cg_status cg_spmm_device(const cg_hamiltonian* h, const void* x, int32_t ldx, void* y, int32_t ldy, int32_t m,
                          int32_t precision);
 
