@@ -762,7 +762,7 @@ cg_status cg_spmm_set_tiled_shape(cg_hamiltonian* h, int32_t slices_per_warp, in
     if (slices_per_warp < 1 || slices_per_warp > 4) throw cg::Error(CG_ERR_ARG, "slices per warp must be 1..4");
     const int warps = (t->smax + slices_per_warp - 1) / slices_per_warp;
     if (warps > 31) throw cg::Error(CG_ERR_ARG, "more than 31 consumer warps; take more slices per warp");
-    if (stages < 2 || stages > 7 || cg::tiled_smem(*t, stages) > 227 * 1024)
+    if (stages < 2 || stages > 7 || cg::tiled_smem(*t, stages) > cg::kSmemMax)
       throw cg::Error(CG_ERR_ARG, "ring slots out of range (2..7 within 227 KB of shared memory)");
     t->rps = slices_per_warp;
     t->warps = warps;

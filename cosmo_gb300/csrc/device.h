@@ -22,6 +22,12 @@ namespace cg {
                             std::to_string(__LINE__) + ")");                                     \
   } while (0)
 
+// Dynamic shared memory a kernel without static shared memory may ask for.  The
+// attribute belongs to the function and the last caller's value holds: a kernel
+// whose size depends on the handle gets this limit from everyone, since a
+// smaller value would refuse the launch of another thread's larger handle.
+constexpr int kSmemMax = 227 * 1024;
+
 // Kernel launches issued by this library (for benchmark accounting).
 uint64_t& launch_counter();
 inline void count_launch(uint64_t k = 1) { launch_counter() += k; }

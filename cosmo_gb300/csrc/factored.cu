@@ -554,7 +554,7 @@ std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op
   // at least 16 spectators a chunk beside the largest matrix
   f.smem32 = std::max(kFSmem, int(sizeof(FHead32)) + f.dmax * fact_tiles(f.dmax) * 64 +
                                   16 * (f.dmax * 36 + 2 * f.cols * 4));
-  if (f.smem32 > 227 * 1024) return nullptr;
+  if (f.smem32 > kSmemMax) return nullptr;
   // few jobs: split their spectators (whole tiles of 16, or 64 rows) until there are some per CTA slot
   constexpr size_t kEnough = 152 * 16;
   for (uint32_t kind = 0; kind < 2; ++kind) {
@@ -615,7 +615,7 @@ void factored_product_f32(const FactoredOp& f, const float* x, float* y, int ldy
   if (!f.n) return;
   FArgs a{f.n, f.cols, f.jobs.p, f.list.p, f.stab.p, f.spect.p};
   const unsigned char* xb = reinterpret_cast<const unsigned char*>(x);
-  CG_CUDA(cudaFuncSetAttribute(k_fact32, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem32));
+  CG_CUDA(cudaFuncSetAttribute(k_fact32, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
   k_fact32<<<unsigned(f.njobs_pn), kFW * 32, f.smem32, s>>>(a, f.wf.p, xb, f.z.p, f.smem32);
   CG_CUDA(cudaGetLastError());
   count_launch();

@@ -580,9 +580,10 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
   int L = 1;
   while (!tab && L < h.max_row) L <<= 1;
   size_t smem = size_t(L) * 16;
-  if (smem > 200 * 1024) throw Error(CG_ERR_UNSUPPORTED, "row longer than the per-row sort supports");
+  constexpr int kSmemSort = 200 * 1024;  // beside the kernel's static shared memory
+  if (smem > kSmemSort) throw Error(CG_ERR_UNSUPPORTED, "row longer than the per-row sort supports");
   if (smem > 48 * 1024)
-    CG_CUDA(cudaFuncSetAttribute(k_sort_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    CG_CUDA(cudaFuncSetAttribute(k_sort_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSort));
   DBuf<unsigned long long> dup(1);
   CG_CUDA(cudaMemsetAsync(dup.p, 0, 8, s));
   if (tab) {

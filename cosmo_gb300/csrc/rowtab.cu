@@ -284,6 +284,7 @@ __device__ __forceinline__ double p1_value(const Ctx& c, const Entry& e, uint32_
 // general builder takes 5.0 + 7.2 ms and 8.1 ms to sort the rows; bound by the
 // lookups of the two-body table and by lists of unequal length in a warp.
 constexpr int kRowsPerWarp = 8;
+constexpr size_t kSmemRow = 200 * 1024;  // of a CTA's rows
 template <bool COUNT>
 __global__ void __launch_bounds__(256) k_rows(Ctx c, Lists l, uint32_t* __restrict__ counts, int cap,
                                               const uint64_t* __restrict__ rowptr, uint32_t* __restrict__ col,
@@ -519,11 +520,11 @@ struct Impl : RowTables {
     CG_CUDA(cudaMemcpyAsync(&m, longest.p, sizeof(m), cudaMemcpyDeviceToHost, s));
     CG_CUDA(cudaStreamSynchronize(s));
     cap = int((m + 1) & ~1u);
-    return smem() <= 200 * 1024;
+    return smem() <= kSmemRow;
   }
   void fill(const uint64_t* rowptr, uint32_t* col, double* out64, float* hi, float* lo, double* dg,
             unsigned long long* upper) override {
-    CG_CUDA(cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem())));
+    CG_CUDA(cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     k_rows<false><<<grid(), 256, smem(), s>>>(c, l, nullptr, cap, rowptr, col, out64, hi, lo, diag.p, upper, nullptr);
     CG_CUDA(cudaGetLastError());
     count_launch();

@@ -625,7 +625,7 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
     for (int rps : {1, 2, 3})
       for (int st : {2, 3, 4, 6}) {
         if ((t.smax + rps - 1) / rps > 31) continue;  // at most 31 consumer warps
-        if (tiled_smem(t, st) > 227 * 1024) continue;
+        if (tiled_smem(t, st) > kSmemMax) continue;
         t.rps = rps;
         t.warps = (t.smax + rps - 1) / rps;
         t.stages = st;

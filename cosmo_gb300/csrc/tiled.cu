@@ -483,7 +483,7 @@ void launch_tiled(const TiledOp& t, const TArgs& a, const float* x, float* y, in
                   cudaStream_t s) {
   const size_t smem = tiled_smem(t, t.stages);
   const int nw = (t.smax + RPS - 1) / RPS;
-  CG_CUDA(cudaFuncSetAttribute(k_tiled<RPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  CG_CUDA(cudaFuncSetAttribute(k_tiled<RPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
   k_tiled<RPS><<<unsigned(t.nb), (nw + 1) * 32, smem, s>>>(a, x, y, ldy, m, err);
   CG_CUDA(cudaGetLastError());
   count_launch();
@@ -664,7 +664,7 @@ void tiled_product(const Hamiltonian& h, const float* x, float* y, int ldy, int 
   const TiledOp& t = *h.tiled;
   if (m < 1 || m > 8) throw Error(CG_ERR_ARG, "tiled product takes 1..8 vectors");
   if (reinterpret_cast<uintptr_t>(x) % 16) throw Error(CG_ERR_ARG, "tiled product needs a 16-byte aligned x");
-  if (t.stages < 2 || 2 * t.stages * 8 + 4 > kTiledHead || tiled_smem(t, t.stages) > 227 * 1024)
+  if (t.stages < 2 || 2 * t.stages * 8 + 4 > kTiledHead || tiled_smem(t, t.stages) > kSmemMax)
     throw Error(CG_ERR_ARG, "tiled product: ring slots out of range");
   TArgs a{t.bstart.p, t.order.p, t.iptr.p, reinterpret_cast<const TItem*>(t.items.p), t.rcopy.p, t.col.p, t.val.p,
           t.dptr.p, reinterpret_cast<const uint2*>(t.iden.p), t.lmax, t.gmax, t.stages};

@@ -474,7 +474,7 @@ template <class T, int VB, int RPT, bool DF, bool TR, class M, bool ST>
 void launch_rpt(const Hamiltonian& h, const VArgs& a, const VTab<T>& tb, const VTab<T>& tl, const T* x, void* y,
                 int ldy, int m, int threads, size_t smem, int* err, cudaStream_t s) {
   auto kern = k_virtual<T, VB, RPT, DF, TR, M, ST>;
-  CG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  CG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
   kern<<<unsigned(a.lmax ? h.virt->nblocks : 0), threads, smem, s>>>(a, tb, tl, x, y, ldy, m, err);
   CG_CUDA(cudaGetLastError());
   count_launch();
@@ -516,9 +516,9 @@ void virtual_product(const Hamiltonian& h, const T* x, void* y, int ldy, int m, 
   const size_t tabs = (3 * size_t(npp + 4) + 2 * size_t(v.np)) * vsz;
   const size_t smem_staged = kVirtualSmemHead + size_t(3) * v.lmax * VB * sizeof(T) + tabs +
                              (v.truncated ? 16 + size_t(3) * v.rmax * sizeof(uint16_t) : 0);
-  const bool staged = smem_staged <= 227 * 1024;
+  const bool staged = smem_staged <= kSmemMax;
   const size_t smem = staged ? smem_staged : kVirtualSmemHead + tabs + 16;
-  if (smem > 227 * 1024) throw Error(CG_ERR_UNSUPPORTED, "interaction slices too large for shared memory");
+  if (smem > kSmemMax) throw Error(CG_ERR_UNSUPPORTED, "interaction slices too large for shared memory");
   // rows per thread: threads <= 512, or <= 1024 when the staging buffers
   // leave room for one CTA per SM only (long blocks, e.g. fp 5+5): there two
   // rows per thread and twice the warps hide the shared-memory latency better
