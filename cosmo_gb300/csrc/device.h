@@ -16,10 +16,12 @@ namespace cg {
 #define CG_CUDA(call)                                                                            \
   do {                                                                                           \
     cudaError_t e_ = (call);                                                                     \
-    if (e_ != cudaSuccess)                                                                       \
+    if (e_ != cudaSuccess) {                                                                     \
+      cudaGetLastError(); /* reported here, not by the check of a later launch */                \
       throw ::cg::Error(e_ == cudaErrorMemoryAllocation ? CG_ERR_NOMEM : CG_ERR_CUDA,            \
                         std::string(#call) + ": " + cudaGetErrorString(e_) + " (" __FILE__ ":" + \
                             std::to_string(__LINE__) + ")");                                     \
+    }                                                                                            \
   } while (0)
 
 // Dynamic shared memory a kernel without static shared memory may ask for.  The

@@ -480,37 +480,36 @@ struct Impl : RowTables {
   DBuf<unsigned> longest;
   int cap = 0;  // longest row before the drops (after count)
 
-  // list starts from counts (host scan: a few thousand lists)
-  uint64_t starts(const DBuf<uint32_t>& cnt, uint64_t k, DBuf<uint64_t>& off) {
+  // list starts from counts (host scan); uses += entries x rows that read them
+  template <class W>
+  uint64_t starts(const DBuf<uint32_t>& cnt, uint64_t k, DBuf<uint64_t>& off, W&& rows, uint64_t& uses) {
     std::vector<uint32_t> h(k);
     CG_CUDA(cudaMemcpyAsync(h.data(), cnt.p, k * 4, cudaMemcpyDeviceToHost, s));
     CG_CUDA(cudaStreamSynchronize(s));
     std::vector<uint64_t> o(k + 1, 0);
-    for (uint64_t i = 0; i < k; ++i) o[i + 1] = o[i] + h[i];
+    for (uint64_t i = 0; i < k; ++i) {
+      o[i + 1] = o[i] + h[i];
+      uses += h[i] * rows(i);
+    }
     off.upload(o, s);
     CG_CUDA(cudaStreamSynchronize(s));  // o leaves
     return o[k];
   }
-  template <class F, class G>
-  void lists(uint64_t k, DBuf<uint64_t>& off, DBuf<Entry>& out, F&& count, G&& fill) {
-    DBuf<uint32_t> cnt(std::max<uint64_t>(k, 1));
-    count(cnt.p);
-    CG_CUDA(cudaGetLastError());
-    const uint64_t total = starts(cnt, k, off);
+  template <class G>
+  void lists(uint64_t k, uint64_t total, const DBuf<uint64_t>& off, DBuf<Entry>& out, G&& fill) {
     DBuf<Entry> raw(std::max<uint64_t>(total, 1));
     out.alloc(std::max<uint64_t>(total, 1));
     fill(off.p, raw.p);
     CG_CUDA(cudaGetLastError());
     k_order<<<unsigned((k * 32 + 255) / 256), 256, 0, s>>>(k, off.p, raw.p, out.p);
     CG_CUDA(cudaGetLastError());
-    count_launch(3);
+    count_launch(2);
     CG_CUDA(cudaStreamSynchronize(s));  // raw leaves
   }
 
   size_t smem() const { return size_t(8) * cap * 12; }
   unsigned grid() const { return unsigned((c.n + 8 * kRowsPerWarp - 1) / (8 * kRowsPerWarp)); }
   bool count(uint32_t* counts) override {
-    longest.alloc(1);
     CG_CUDA(cudaMemsetAsync(longest.p, 0, sizeof(unsigned), s));
     k_rows<true><<<grid(), 256, 0, s>>>(c, l, counts, 0, nullptr, nullptr, nullptr, nullptr, nullptr, diag.p, nullptr,
                                         longest.p);
@@ -532,9 +531,7 @@ struct Impl : RowTables {
   }
 };
 
-}  // namespace
-
-std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cudaStream_t s) {
+std::unique_ptr<RowTables> make_tables(const Basis& b, const DevOperator& op, cudaStream_t s) {
   if (b.wide || b.truncated || !b.n || b.n >= (1ull << 32) || b.ns > kMaxNs) return nullptr;
   // one parity per species and half-integer (or integer) 2m throughout: the
   // change of 2m alone then pairs neutron and proton moves
@@ -553,7 +550,19 @@ std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cud
   c.npairs = op.npairs;
   c.n = b.n;
   c.nblocks = int(b.h_bstart.size());
-  c.nconf = b.h_cmasks.size();
+  // the proton configurations of the classes that some block uses, class by class
+  const size_t nclass = b.h_cstart.size();
+  const auto class_end = [&](size_t i) { return i + 1 < nclass ? b.h_cstart[i + 1] : uint32_t(b.h_cmasks.size()); };
+  std::vector<uint64_t> blocks(nclass, 0);  // of each class
+  for (uint32_t k : b.h_bclass) ++blocks[k];
+  std::vector<uint32_t> cstart(nclass, 0), cmask, of;
+  for (size_t i = 0; i < nclass; ++i) {
+    cstart[i] = uint32_t(cmask.size());
+    if (!blocks[i]) continue;
+    cmask.insert(cmask.end(), b.h_cmasks.begin() + b.h_cstart[i], b.h_cmasks.begin() + class_end(i));
+    of.resize(cmask.size(), uint32_t(i));
+  }
+  c.nconf = cmask.size();
   for (int i = 0; i < b.ns; ++i) c.m2max = std::max(c.m2max, std::abs(b.sp_m2[i]));
   c.ndm = 2 * c.m2max + 1;
   c.dm0 = c.m2max;
@@ -562,8 +571,8 @@ std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cud
   t->bstart.upload(b.h_bstart, s);
   t->bmask.upload(b.h_bmask, s);
   t->bclass.upload(b.h_bclass, s);
-  t->cstart.upload(b.h_cstart, s);
-  t->cmask.upload(b.h_cmasks, s);
+  t->cstart.upload(cstart, s);
+  t->cmask.upload(cmask, s);
   std::vector<int8_t> m2(b.sp_m2.begin(), b.sp_m2.end());
   t->m2.upload(m2, s);
   c.noff = b.noff.p;
@@ -578,14 +587,30 @@ std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cud
   c.cmask = t->cmask.p;
   c.m2 = t->m2.p;
   const unsigned gb = unsigned((c.nblocks + 63) / 64), gc = unsigned((c.nconf + 63) / 64);
-  t->lists(c.nblocks, t->noff, t->nl, [&](uint32_t* k) { k_nlist<false><<<gb, 64, 0, s>>>(c, k, nullptr, nullptr); },
-           [&](const uint64_t* o, Entry* e) { k_nlist<true><<<gb, 64, 0, s>>>(c, nullptr, o, e); });
-  t->lists(c.nconf, t->ooff, t->ol, [&](uint32_t* k) { k_olist<false><<<gc, 64, 0, s>>>(c, k, nullptr, nullptr); },
-           [&](const uint64_t* o, Entry* e) { k_olist<true><<<gc, 64, 0, s>>>(c, nullptr, o, e); });
-  t->pt.alloc(std::max<uint64_t>(c.nconf * c.tp, 1));
-  t->poff.alloc(c.nconf * (c.ndm + 1));
-  k_plist<<<unsigned((c.nconf * 32 + 255) / 256), 256, size_t(c.tp) * 8 * sizeof(uint2), s>>>(c, t->pt.p, t->poff.p);
+  DBuf<uint32_t> ncnt(std::max(c.nblocks, 1)), ocnt(std::max<uint64_t>(c.nconf, 1));
+  k_nlist<false><<<gb, 64, 0, s>>>(c, ncnt.p, nullptr, nullptr);
   CG_CUDA(cudaGetLastError());
+  k_olist<false><<<gc, 64, 0, s>>>(c, ocnt.p, nullptr, nullptr);
+  CG_CUDA(cudaGetLastError());
+  count_launch(2);
+  uint64_t uses = 0;
+  const uint64_t nls = t->starts(ncnt, c.nblocks, t->noff,
+                                 [&](uint64_t i) { return uint64_t(class_end(b.h_bclass[i])) - b.h_cstart[b.h_bclass[i]]; },
+                                 uses);
+  const uint64_t ols = t->starts(ocnt, c.nconf, t->ooff, [&](uint64_t g) { return blocks[of[g]]; }, uses);
+  const uint64_t moves = c.kn ? c.nconf * (c.tp * sizeof(uint2) + (c.ndm + 1) * sizeof(uint16_t)) : 0;
+  if (!row_tables_worth((nls + ols) * 2 * sizeof(Entry) + moves, uses)) return nullptr;
+  t->lists(c.nblocks, nls, t->noff, t->nl,
+           [&](const uint64_t* o, Entry* e) { k_nlist<true><<<gb, 64, 0, s>>>(c, nullptr, o, e); });
+  t->lists(c.nconf, ols, t->ooff, t->ol,
+           [&](const uint64_t* o, Entry* e) { k_olist<true><<<gc, 64, 0, s>>>(c, nullptr, o, e); });
+  if (c.kn) {  // else no neutron moves, and nothing reads them
+    t->pt.alloc(std::max<uint64_t>(c.nconf * c.tp, 1));
+    t->poff.alloc(c.nconf * (c.ndm + 1));
+    k_plist<<<unsigned((c.nconf * 32 + 255) / 256), 256, size_t(c.tp) * 8 * sizeof(uint2), s>>>(c, t->pt.p, t->poff.p);
+    CG_CUDA(cudaGetLastError());
+    count_launch();
+  }
   const int words = (c.np * c.np + 31) / 32;
   t->nz.alloc(std::max(c.nn * c.nn * words, 1));
   if (c.nn && c.np) {
@@ -596,9 +621,21 @@ std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cud
   t->diag.alloc(c.n);
   k_diagonal<<<unsigned((c.n + 255) / 256), 256, 0, s>>>(c, b.state.p, t->diag.p);
   CG_CUDA(cudaGetLastError());
-  count_launch(2);
+  count_launch();
+  t->longest.alloc(1);
   t->l = Lists{t->noff.p, t->ooff.p, t->nl.p, t->ol.p, t->pt.p, t->poff.p, t->nz.p, words};
   return t;
+}
+
+}  // namespace
+
+std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cudaStream_t s) {
+  try {
+    return make_tables(b, op, s);
+  } catch (const Error& e) {
+    if (e.code != CG_ERR_NOMEM) throw;
+    return nullptr;  // what was allocated is free again; the general builder needs no tables
+  }
 }
 
 }  // namespace cg

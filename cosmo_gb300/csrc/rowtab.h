@@ -23,6 +23,13 @@ struct RowTables {
   virtual void fill(const uint64_t* rowptr, uint32_t* col, double* out64, float* hi, float* lo, double* diag,
                     unsigned long long* upper) = 0;
 };
+// Whether tables of `bytes` (while they are made; about half afterwards) pay
+// whose entries are read `uses` times by all rows together.  With one species
+// moving the lists are as long as the rows themselves and no two rows share one
+// (30 states, 10 protons: 32 bytes for each of 7e8 elements), and the general
+// builder, whose unsorted values take 8 bytes an element, needs less memory.
+constexpr uint64_t kRowTableBytes = 1ull << 30;
+inline bool row_tables_worth(uint64_t bytes, uint64_t uses) { return bytes <= kRowTableBytes + 8 * uses; }
 std::unique_ptr<RowTables> row_tables(const Basis& b, const DevOperator& op, cudaStream_t s);
 
 }  // namespace cg
