@@ -739,7 +739,7 @@ cg_status cg_spmm_set_format(cg_hamiltonian* h, int32_t format) {
     CG_NOT_NULL(h);
     if (format != CG_FORMAT_ROWS && format != CG_FORMAT_TILED && format != CG_FORMAT_FACTORED)
       throw cg::Error(CG_ERR_ARG, "unknown SpMM format");
-    if (format == CG_FORMAT_FACTORED && (!h->h.fact || h->h.virt))
+    if (format == CG_FORMAT_FACTORED && !h->h.fact)
       throw cg::Error(CG_ERR_UNSUPPORTED, "no factored form of this matrix");
     if (format == CG_FORMAT_TILED && !h->h.tiled && !h->h.virt && h->h.precision == CG_PREC_FP32 &&
         !h->h.blocks.empty()) {
@@ -771,7 +771,6 @@ cg_status cg_spmm_set_tiled_shape(cg_hamiltonian* h, int32_t slices_per_warp, in
 }
 
 static int32_t format_in_use(const cg::Hamiltonian& h) {
-  if (h.virt) return CG_FORMAT_ROWS;
   return h.use_fact() ? CG_FORMAT_FACTORED : h.use_tiled() ? CG_FORMAT_TILED : CG_FORMAT_ROWS;
 }
 

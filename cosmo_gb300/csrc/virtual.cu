@@ -631,7 +631,7 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
 }
 
 void virtual_product_f32(const Hamiltonian& h, const float* x, float* y, int ldy, int m, cudaStream_t s) {
-  if (h.fact) return factored_product_f32(*h.fact, x, y, ldy, m, s);
+  if (h.use_fact()) return factored_product_f32(*h.fact, x, y, ldy, m, s);
   VTab<float> tb{h.virt->Wf.p, h.virt->Unf.p, h.virt->Upf.p, h.virt->sl_cf.p, h.virt->pp_hf.p};
   virtual_product<float, kVirtualVB32>(h, x, y, ldy, m, tb, tb, s);
 }
@@ -1159,6 +1159,7 @@ void virtual_build(const System& sys, const Operator& op, const Basis& b, int pr
   // sd 3 + 3 15 / 49 us; near half filling most pairs of a core are blocked and
   // k_virtual stays (sd 6 + 6 172 / 129 us, sd 8 + 8 149 / 67).
   h.fact = factored_build(sys, op, b, 40 + 3.6e-6 * double(conn), s);
+  if (h.fact) h.format = CG_FORMAT_FACTORED;
   h.virt = vp;
   h.nnz = conn;
   h.nnz_upper = 0;

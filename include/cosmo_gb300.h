@@ -245,7 +245,8 @@ cg_status cg_spmm_get_tuning(const cg_hamiltonian* h, int32_t* warps, int32_t* c
  * Factored: H applied through the determinants with two particles taken out,
  * small dense matrices per core instead of the stored elements; an FP32 matrix
  * of 2^24 stored entries or more, built from an untruncated basis, uses it by
- * default where it is estimated faster.  Block-tiled copy of an FP32 matrix
+ * default where it is estimated faster, and so does an on-the-fly Hamiltonian,
+ * for which CG_FORMAT_ROWS is the element-wise product.  Block-tiled copy of an FP32 matrix
  * built from a basis: tiles = (neutron block, neutron block) pairs, 16-bit
  * in-tile columns, x of the column block staged in shared memory per tile.  The reference's counterpart is its fixed CSB blocking
  * (PPMatrix2CSBBlk, include/sm/PPMatrix.cxx:571-656); the choice of format has
