@@ -15,6 +15,7 @@
 #include "davidson.h"
 #include "dense.h"
 #include "device.h"
+#include "factored.h"
 #include "model.h"
 #include "batched.h"
 #include "tiled.h"
@@ -749,6 +750,13 @@ cg_status cg_spmm_set_format(cg_hamiltonian* h, int32_t format) {
     if (format == CG_FORMAT_TILED && !h->h.tiled)
       throw cg::Error(CG_ERR_UNSUPPORTED,
                       "no block-tiled copy (needs an FP32 matrix built from a basis, blocks <= 1536 rows)");
+    if (format == CG_FORMAT_FACTORED) {
+      CG_CUDA(cudaSetDevice(h->h.device));
+      if (!cg::factored_ready(h->h)) throw cg::Error(CG_ERR_NOMEM, "no memory for the factored form's work area");
+      h->h.fact_failed = false;
+    } else if (h->h.fact) {
+      h->h.fact->z.release();
+    }
     h->h.format = format;
   });
 }

@@ -29,6 +29,7 @@
 
 #include "davidson.h"
 #include "dfloat.h"
+#include "factored.h"
 #include "virtual.h"
 #include "dense.h"
 #include "device.h"
@@ -1710,7 +1711,7 @@ static void store_vectors(Engine<T>& e, int m, double* dst_dev_cm) {
     count_launch();
 }
 
-DavResult davidson_solve(const Hamiltonian& h, const DavidsonRequest& rq) {
+static DavResult solve(const Hamiltonian& h, const DavidsonRequest& rq) {
   cudaStream_t s = h.stream;
   DavResult res;
   const uint64_t n = h.n;
@@ -1760,6 +1761,23 @@ DavResult davidson_solve(const Hamiltonian& h, const DavidsonRequest& rq) {
   res.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   if (rq.vecs_out) CG_CUDA(cudaMemcpy(rq.vecs_out, vecs.p, n * nume * 8, cudaMemcpyDeviceToHost));
   return res;
+}
+
+// The solve's vectors have precedence over what products keep: an on-the-fly
+// matrix gives the factored form's work area back after a solve that took it,
+// and where memory runs out the solve is done over without that area.
+DavResult davidson_solve(const Hamiltonian& h, const DavidsonRequest& rq) {
+  struct Area {
+    const FactoredOp* f;
+    ~Area() { if (f) f->z.release(); }
+  } area{h.virt && h.fact && !h.fact->z.p ? h.fact.get() : nullptr};
+  try {
+    return solve(h, rq);
+  } catch (const Error& e) {
+    if (e.code != CG_ERR_NOMEM || !h.release_work()) throw;
+    h.fact_failed = h.fact != nullptr;
+    return solve(h, rq);
+  }
 }
 
 }  // namespace cg

@@ -213,10 +213,14 @@ struct Hamiltonian {
   mutable DBuf<unsigned char> host_work;  // device buffers of host products (spmm_host)
   std::vector<uint64_t> blocks;     // neutron-block starts (+ n) when built from a basis
   int format = CG_FORMAT_TILED;     // what FP32 products of up to 8 vectors use, where it exists
-  bool use_fact() const { return fact && format == CG_FORMAT_FACTORED; }
+  mutable bool fact_failed = false; // the factored form's work area could not be allocated
+  bool use_fact() const { return fact && format == CG_FORMAT_FACTORED && !fact_failed; }
   bool use_tiled() const { return tiled && format == CG_FORMAT_TILED; }
   cudaStream_t stream = nullptr;
   ~Hamiltonian();
+  // Gives back what products keep between calls (the work area of the factored
+  // form, packed operands, buffers of host products); false when there is nothing.
+  bool release_work() const;
   uint64_t device_bytes() const;  // HBM held by the matrix (or the on-the-fly tables)
 };
 

@@ -367,10 +367,8 @@ Cores make_cores(int norb, int k, const int* m2, const int* par) {
   return out;
 }
 
-}  // namespace
-
-std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op, const Basis& b, double other_us,
-                                           cudaStream_t s) {
+std::shared_ptr<FactoredOp> build_tables(const System& sys, const Operator& op, const Basis& b, double other_us,
+                                         cudaStream_t s) {
   const int nn = b.nn, np = b.np, ns = b.ns, kn = b.kn, kp = b.kp;
   if (b.wide || b.truncated || !b.n || kn < 1 || kp < 1 || nn > 32 || np > 32) return nullptr;
   const int slots = kn * kp + kn * (kn - 1) / 2 + kp * (kp - 1) / 2;
@@ -599,13 +597,32 @@ std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op
   f.spect.upload(spect, s);
   const std::vector<float> wf(w.begin(), w.end());
   f.wf.upload(wf, s);
-  // the work area: at most a quarter of what is free now, else the other product serves
-  size_t avail = 0, total = 0;
-  CG_CUDA(cudaMemGetInfo(&avail, &total));
-  if (uint64_t(slots) * b.n * 32 > avail / 4) return nullptr;
-  f.z.alloc(uint64_t(slots) * b.n * 32);
   CG_CUDA(cudaStreamSynchronize(s));
   return fp;
+}
+
+}  // namespace
+
+std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op, const Basis& b, double other_us,
+                                           cudaStream_t s) {
+  try {
+    return build_tables(sys, op, b, other_us, s);
+  } catch (const Error& e) {
+    if (e.code != CG_ERR_NOMEM) throw;
+    return nullptr;
+  }
+}
+
+bool factored_ready(const Hamiltonian& h) {
+  const FactoredOp& f = *h.fact;
+  if (f.z.p || !f.n) return true;
+  try {
+    f.z.alloc(uint64_t(f.slots) * f.n * 32);
+  } catch (const Error& e) {
+    if (e.code != CG_ERR_NOMEM) throw;
+    h.fact_failed = true;
+  }
+  return f.z.p;
 }
 
 void factored_product_f32(const FactoredOp& f, const float* x, float* y, int ldy, int m, cudaStream_t s) {

@@ -59,7 +59,7 @@ struct FactoredOp {
   DBuf<uint32_t> spect;         // block starts of each proton class
   double est_us = 0;            // estimated time of one product
   DBuf<float> wf;               // channel matrices
-  mutable DBuf<unsigned char> z;  // partial sums: slots x n rows of 32 bytes
+  mutable DBuf<unsigned char> z;  // partial sums: slots x n rows of 32 bytes (factored_ready)
   uint64_t bytes() const {
     return jobs.bytes() + list.bytes() + stab.bytes() + spect.bytes() + wf.bytes() + z.bytes();
   }
@@ -67,8 +67,8 @@ struct FactoredOp {
 
 // Tables of the factored product, or null where it does not apply (a truncated
 // or wide basis, a species without particles, channels, rows or a work area
-// beyond its limits) or is estimated slower than other_us, the time of the
-// product it would replace.
+// beyond its limits), where its tables cannot be allocated, or where it is
+// estimated slower than other_us, the time of the product it would replace.
 std::shared_ptr<FactoredOp> factored_build(const System& sys, const Operator& op, const Basis& b, double other_us,
                                            cudaStream_t s);
 constexpr uint64_t kFactoredMaxWork = 32ull << 30;
@@ -76,8 +76,15 @@ constexpr uint64_t kFactoredMaxWork = 32ull << 30;
 // (fp 2+4, 3.3e7 entries: 120 us row-wise, 60 factored; sd 4+4, 6e6: 24 and 33)
 constexpr uint64_t kFactoredMinEntries = 1ull << 24;
 
+// The matrix's work area is there, or is allocated now.  Where that fails the
+// product that was replaced serves from then on (until cg_spmm_set_format asks
+// for the factored form again).  A stored matrix takes the area when it is
+// built, an on-the-fly one with its first FP32 product: the path is there for
+// problems that fill the device, and a solve's vectors come first.
+bool factored_ready(const Hamiltonian& h);
+
 // Y = H X from x packed as n rows of 8 FP32 vectors (32-byte aligned).
-// Asynchronous; allocates nothing.
+// Asynchronous; allocates nothing (factored_ready has been called).
 void factored_product_f32(const FactoredOp& f, const float* x, float* y, int ldy, int m, cudaStream_t s);
 
 }  // namespace cg

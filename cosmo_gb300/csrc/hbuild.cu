@@ -630,7 +630,8 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
     const double per_block = double(n) / double(std::max<size_t>(b.h_bstart.size(), 1));
     const double per_entry = h.nnz >= kTiledMinEntries ? std::min(3.4e-6, 1.9e-6 * (1 + 40 / per_block)) : 3.4e-6;
     h.fact = factored_build(sys, op, b, 5 + per_entry * double(h.nnz), s);
-    if (h.fact) h.format = CG_FORMAT_FACTORED;
+    if (h.fact && factored_ready(h)) h.format = CG_FORMAT_FACTORED;
+    else h.fact.reset();  // no room for its work area
     h.build_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
   if (precision == CG_PREC_FP32 && tiled_copy && !h.fact && h.nnz >= kTiledMinEntries) {

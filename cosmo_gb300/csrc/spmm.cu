@@ -639,8 +639,8 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
     out.push_back({bw, 0, tbest});
     if (tbest < best) { best = tbest; best_format = CG_FORMAT_TILED; }
   }
-  if (h.fact && m <= 8) {
-    h.format = CG_FORMAT_FACTORED;
+  h.format = CG_FORMAT_FACTORED;
+  if (m <= 8 && h.use_fact() && factored_ready(h)) {
     const float med = time_once();
     out.push_back({0, -1, med});
     if (med < best) { best = med; best_format = CG_FORMAT_FACTORED; }
@@ -788,7 +788,8 @@ void spmm_f32_padded(const Hamiltonian& h, const float* x, int ldx, float* y, in
   if (h.precision != CG_PREC_FP32) throw Error(CG_ERR_ARG, "FP32 product needs an FP32 matrix");
   if (m < 1 || m > 16) throw Error(CG_ERR_ARG, "padded FP32 SpMM takes 1..16 vectors");
   if (reinterpret_cast<uintptr_t>(x) % 32 || ldx % 8) throw Error(CG_ERR_ARG, "padded FP32 SpMM needs 32-byte rows");
-  if (m <= 8 && ldx == 8 && h.use_fact()) return factored_product_f32(*h.fact, x, y, ldy, m, s);
+  if (m <= 8 && ldx == 8 && h.use_fact() && factored_ready(h))
+    return factored_product_f32(*h.fact, x, y, ldy, m, s);
   if (m <= 8 && ldx == 8 && h.use_tiled()) return tiled_product(h, x, y, ldy, m, s);
   if (m <= 8) {
     if (ldx < 8) throw Error(CG_ERR_ARG, "ldx < 8");
@@ -811,7 +812,7 @@ void spmm_launch(const Hamiltonian& h, int precision, const void* x, int ldx, vo
       break;
     case CG_PREC_FP32:
       if (h.precision != CG_PREC_FP32) throw Error(CG_ERR_ARG, "FP32 product needs an FP32 matrix");
-      if (m <= 8 && ldx == 8 && h.use_fact() && reinterpret_cast<uintptr_t>(x) % 32 == 0)
+      if (m <= 8 && ldx == 8 && reinterpret_cast<uintptr_t>(x) % 32 == 0 && h.use_fact() && factored_ready(h))
         return factored_product_f32(*h.fact, static_cast<const float*>(x), static_cast<float*>(y), ldy, m, s);
       if (m <= 8 && ldx == 8 && h.use_tiled() && reinterpret_cast<uintptr_t>(x) % 16 == 0)
         return tiled_product(h, static_cast<const float*>(x), static_cast<float*>(y), ldy, m, s);

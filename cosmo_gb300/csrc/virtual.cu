@@ -591,8 +591,13 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
   if (m < 1) throw Error(CG_ERR_ARG, "m must be >= 1");
   if (ldx < m || ldy < m) throw Error(CG_ERR_ARG, "leading dimension smaller than the vector count");
   const uint64_t n = h.n;
-  // n packed rows of 32 bytes in every precision, kept with the handle
-  const DBuf<unsigned char>& pack = h.virt->pack;
+  // n packed rows of 32 bytes in every precision, kept with the handle from the
+  // first call that packs
+  DBuf<unsigned char>& pack = h.virt->pack;
+  const auto packed_rows = [&] {
+    if (pack.n < n * 32) pack.alloc(n * 32);
+    return pack.p;
+  };
   // Rows that are packed already are taken as they are, unless y overlaps them:
   // a CTA of the product gathers rows of x whose y another CTA writes.
   const auto direct = [&](int mc, int vb, size_t elem) {
@@ -601,29 +606,35 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
     return mc == vb && ldx == vb && x0 % 32 == 0 && (y1 <= x0 || x1 <= y0);
   };
   if (precision == CG_PREC_FP32) {
-    float* w = reinterpret_cast<float*>(pack.p);
     const float* xf = static_cast<const float*>(x);
     for (int c0 = 0; c0 < m; c0 += kVirtualVB32) {
       const int mc = std::min(kVirtualVB32, m - c0);
-      const bool packed = direct(mc, kVirtualVB32, sizeof(float));
-      if (!packed) virtual_pack_f32(n, xf, ldx, c0, mc, w, s);
-      virtual_product_f32(h, packed ? xf : w, static_cast<float*>(y) + c0, ldy, mc, s);
+      const float* w = xf;
+      if (!direct(mc, kVirtualVB32, sizeof(float))) {
+        float* t = reinterpret_cast<float*>(packed_rows());
+        virtual_pack_f32(n, xf, ldx, c0, mc, t, s);
+        w = t;
+      }
+      virtual_product_f32(h, w, static_cast<float*>(y) + c0, ldy, mc, s);
     }
   } else if (precision == CG_PREC_REFINE) {
-    float* w = reinterpret_cast<float*>(pack.p);
+    float* w = reinterpret_cast<float*>(packed_rows());
     for (int c0 = 0; c0 < m; c0 += 4) {
       const int mc = std::min(4, m - c0);
       virtual_pack_df(n, static_cast<const double*>(x), ldx, c0, mc, w, s);
       virtual_product_df(h, w, static_cast<double*>(y) + c0, ldy, mc, s);
     }
   } else if (precision == CG_PREC_FP64) {
-    double* w = reinterpret_cast<double*>(pack.p);
     const double* xd = static_cast<const double*>(x);
     for (int c0 = 0; c0 < m; c0 += kVirtualVB64) {
       const int mc = std::min(kVirtualVB64, m - c0);
-      const bool packed = direct(mc, kVirtualVB64, sizeof(double));
-      if (!packed) virtual_pack_f64(n, xd, ldx, c0, mc, w, s);
-      virtual_product_f64(h, packed ? xd : w, static_cast<double*>(y) + c0, ldy, mc, s);
+      const double* w = xd;
+      if (!direct(mc, kVirtualVB64, sizeof(double))) {
+        double* t = reinterpret_cast<double*>(packed_rows());
+        virtual_pack_f64(n, xd, ldx, c0, mc, t, s);
+        w = t;
+      }
+      virtual_product_f64(h, w, static_cast<double*>(y) + c0, ldy, mc, s);
     }
   } else {
     throw Error(CG_ERR_ARG, "unknown precision");
@@ -631,7 +642,7 @@ void virtual_launch(const Hamiltonian& h, int precision, const void* x, int ldx,
 }
 
 void virtual_product_f32(const Hamiltonian& h, const float* x, float* y, int ldy, int m, cudaStream_t s) {
-  if (h.use_fact()) return factored_product_f32(*h.fact, x, y, ldy, m, s);
+  if (h.use_fact() && factored_ready(h)) return factored_product_f32(*h.fact, x, y, ldy, m, s);
   VTab<float> tb{h.virt->Wf.p, h.virt->Unf.p, h.virt->Upf.p, h.virt->sl_cf.p, h.virt->pp_hf.p};
   virtual_product<float, kVirtualVB32>(h, x, y, ldy, m, tb, tb, s);
 }
@@ -667,6 +678,20 @@ void virtual_pack_df(uint64_t n, const double* x, int ld, int c0, int m, float* 
   k_pack_df<<<unsigned((n * 4 + 255) / 256), 256, 0, s>>>(n, x, ld, c0, m, w);
   CG_CUDA(cudaGetLastError());
   count_launch();
+}
+
+bool Hamiltonian::release_work() const {
+  bool any = host_work.p != nullptr;
+  host_work.release();
+  if (fact) {
+    any |= fact->z.p != nullptr;
+    fact->z.release();
+  }
+  if (virt) {
+    any |= virt->pack.p != nullptr;
+    virt->pack.release();
+  }
+  return any;
 }
 
 uint64_t Hamiltonian::device_bytes() const {
@@ -1151,14 +1176,14 @@ void virtual_build(const System& sys, const Operator& op, const Basis& b, int pr
   }
   CG_CUDA(cudaStreamSynchronize(s));
   v.err.alloc(1);
-  v.pack.alloc(b.n * 32);
   // FP32 products: the factored form where it is estimated faster than k_virtual
   // (40 us of launch and error read-back + 3.6 us per million elements for 8
   // vectors, within 20 % from sd 4 + 4 to fp 4 + 4).  8 vectors, factored /
   // k_virtual: fp 4 + 4 1.36 / 4.34 ms, fp 5 + 3 1.02 / 3.75, fp 3 + 3 0.07 / 0.26,
   // sd 3 + 3 15 / 49 us; near half filling most pairs of a core are blocked and
   // k_virtual stays (sd 6 + 6 172 / 129 us, sd 8 + 8 149 / 67).
-  h.fact = factored_build(sys, op, b, 40 + 3.6e-6 * double(conn), s);
+  // A handle made for FP64 products has no use for it.
+  if (precision == CG_PREC_FP32) h.fact = factored_build(sys, op, b, 40 + 3.6e-6 * double(conn), s);
   if (h.fact) h.format = CG_FORMAT_FACTORED;
   h.virt = vp;
   h.nnz = conn;

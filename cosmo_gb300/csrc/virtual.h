@@ -82,7 +82,7 @@ struct VirtualOp {
   DBuf<uint16_t> lmap;                              // per list: class rank -> list rank
   DBuf<uint32_t> lmap_off, lmap_len;                // lists: first entry, entries (16-byte multiples)
   mutable DBuf<int> err;                            // staged-copy timeout flag
-  DBuf<unsigned char> pack;                         // packed operand of virtual_launch, n x 32 bytes
+  mutable DBuf<unsigned char> pack;                         // packed operand of virtual_launch, n x 32 bytes
   uint64_t bytes() const {
     return bstart.bytes() + blen.bytes() + bclass.bytes() + bmask.bytes() + order.bytes() + cstart.bytes() +
            cmask.bytes() + nt_off.bytes() + nt.bytes() + nn_off.bytes() + nn2.bytes() + cslice.bytes() +

@@ -165,8 +165,9 @@ cg_status cg_hamiltonian_build(const cg_problem* p, const cg_basis* b, int32_t p
  * configurations of each neutron block, targets outside the basis dropped as
  * the reference's locate drops them).  The handle works with every product
  * and Davidson call: CG_PREC_FP32 products compute in FP32, CG_PREC_FP64 and
- * CG_PREC_REFINE products in FP64; precision only sets the default of
- * cg_spmm calls.  info.nnz_full = elements generated per product and vector,
+ * CG_PREC_REFINE products in FP64; precision sets the default of cg_spmm calls
+ * and, for CG_PREC_FP32, lets FP32 products use the factored form (see
+ * cg_spmm_set_format).  info.nnz_full = elements generated per product and vector,
  * info.nnz_upper = 0; cg_hamiltonian_upper_rows / write_hh are unsupported. */
 cg_status cg_hamiltonian_build_virtual(const cg_problem* p, const cg_basis* b, int32_t precision,
                                        cg_hamiltonian** out);
@@ -246,7 +247,12 @@ cg_status cg_spmm_get_tuning(const cg_hamiltonian* h, int32_t* warps, int32_t* c
  * small dense matrices per core instead of the stored elements; an FP32 matrix
  * of 2^24 stored entries or more, built from an untruncated basis, uses it by
  * default where it is estimated faster, and so does an on-the-fly Hamiltonian,
- * for which CG_FORMAT_ROWS is the element-wise product.  Block-tiled copy of an FP32 matrix
+ * of precision CG_PREC_FP32, for which CG_FORMAT_ROWS is the element-wise
+ * product.  It needs a work area of 32 bytes per row and pair of particles (fp
+ * 5+5, 18,600,516 rows: 26.8 GB; at most 32 GiB): taken when a stored matrix is
+ * built, with the first FP32 product of an on-the-fly one (a solve that takes it
+ * gives it back); where it cannot be allocated the other product serves.
+ * Choosing another format frees it.  Block-tiled copy of an FP32 matrix
  * built from a basis: tiles = (neutron block, neutron block) pairs, 16-bit
  * in-tile columns, x of the column block staged in shared memory per tile.  The reference's counterpart is its fixed CSB blocking
  * (PPMatrix2CSBBlk, include/sm/PPMatrix.cxx:571-656); the choice of format has
