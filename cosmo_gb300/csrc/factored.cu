@@ -9,6 +9,7 @@
 // core lacks, so the partial sums need no atomics and k_fsum adds them in a
 // fixed order: the product is deterministic.
 #include <algorithm>
+#include <cmath>
 #include <map>
 
 #include "factored.h"
@@ -19,6 +20,7 @@ namespace {
 
 constexpr int kFMaxPairs = 128;  // pairs of a channel
 constexpr int kFSmem = 56 * 1024;
+constexpr double kFDrop = 1e-14;  // smaller elements are zeros, as in a stored matrix
 
 struct FArgs {
   uint64_t n;
@@ -83,6 +85,43 @@ struct alignas(16) FHead32 {
   uint32_t meta[kFMaxPairs];
 };
 
+// Infinities and NaN.  The channel's matrix is dense, so a row of x that is not
+// finite would turn every output of its cores into NaN through the zeros of the
+// matrix, where the element-wise products reach connected rows only.  It shows
+// in any one output: where that is not finite, all are formed again without the
+// zeros (an infinity still comes out as NaN where the terms of an element differ
+// in sign).
+template <int N>
+__device__ __forceinline__ bool not_finite(const float2 (&v)[N]) {
+  float2 c = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < N; ++i) fma2(c, v[i], make_float2(0.f, 0.f));
+  return !(c.x + c.y == 0.f);
+}
+
+// Output o of a tile's spectator once more, without the zeros of its matrix column wp
+__device__ __noinline__ void redo_row(const FArgs& a, const FHead32& hd, int o, int D, const float* wp, int wld,
+                                      const float4* xp, const uint32_t* sp, int ld, const uint32_t* of,
+                                      unsigned char* z) {
+  const uint32_t at = of[hd.src[o].y];
+  if (at == ~0u) return;
+  float2 acc[4] = {};
+  for (int k = 0; k < D; ++k) {
+    const float w = __uint_as_float(__float_as_uint(wp[k * wld]) ^ sp[k * ld]);
+    if (w == 0.f) continue;
+    const float4 x0 = xp[2 * ld * k], x1 = xp[2 * ld * k + ld];
+    const float2 w2 = make_float2(w, w), xv[4] = {{x0.x, x0.y}, {x0.z, x0.w}, {x1.x, x1.y}, {x1.z, x1.w}};
+    for (int v = 0; v < 4; ++v) fma2(acc[v], w2, xv[v]);
+  }
+  const uint64_t row = hd.dst[o] + (at & kFOff) + uint64_t(at >> kFPosBit) * a.n;
+  Row32 r;
+  for (int v = 0; v < 4; ++v) {
+    r.v[2 * v] = __float_as_uint(acc[v].x) ^ pos_phase(at);
+    r.v[2 * v + 1] = __float_as_uint(acc[v].y) ^ pos_phase(at);
+  }
+  st_row(z + row * 32, r);
+}
+
 // One warp tile: acc += matrix rows x gathered rows, then the output rows.  sg
 // holds the spectator's phase of each (pair, spectator) as a sign bit, applied
 // to the matrix values while they are doubled for the packed multiply-adds.
@@ -120,6 +159,7 @@ __device__ __forceinline__ void tile32(const FArgs& a, const FHead32& hd, int D,
     sp += ld;
   }
   if (!live) return;
+  const bool bad = not_finite(acc[0]);
 #pragma unroll
   for (int t = 0; t < OT; ++t) {
     const int k = group * OT + t;
@@ -138,6 +178,9 @@ __device__ __forceinline__ void tile32(const FArgs& a, const FHead32& hd, int D,
       }
     }
   }
+  if (bad)
+    for (int t = 0; t < OT && group * OT + t < D; ++t)
+      redo_row(a, hd, group * OT + t, D, ws + group * 8 + t, wld, xs + j, sg + j, ld, of, z);
 }
 
 // Outputs of a job in 1, 2 or 4 warp tiles (more above 64 pairs) of 2 groups of
@@ -239,6 +282,22 @@ __global__ void __launch_bounds__(kFW * 32, 4) k_fact32(FArgs a, const float* __
 // another, so nothing but the matrix (phases folded in) is staged.
 constexpr int kFPairs = 32;  // pairs of a one-species job
 
+// a spectator's outputs once more (16-byte halves of the rows), without the zeros of the matrix
+__device__ __noinline__ void redo_half(int D, const uint32_t* src, const uint64_t* dst, const float* ws,
+                                       const unsigned char* x, unsigned char* z, uint32_t off) {
+  for (int o = 0; o < D; ++o) {
+    float2 acc[2] = {};
+    for (int k = 0; k < D; ++k) {
+      const float w = ws[o * kFPairs + k];
+      if (w == 0.f) continue;
+      const float4 r = __ldg(reinterpret_cast<const float4*>(x + uint64_t(src[k] + off) * 32));
+      fma2(acc[0], make_float2(w, w), make_float2(r.x, r.y));
+      fma2(acc[1], make_float2(w, w), make_float2(r.z, r.w));
+    }
+    *reinterpret_cast<float4*>(z + (dst[o] + off) * 32) = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
+  }
+}
+
 template <int DM>
 __device__ __forceinline__ void pairs32(const FArgs& a, const FJob& job, int D, const uint32_t* src,
                                         const uint64_t* dst, const float* ws, const unsigned char* __restrict__ x,
@@ -254,6 +313,7 @@ __device__ __forceinline__ void pairs32(const FArgs& a, const FJob& job, int D, 
       xv[k][0] = make_float2(r.x, r.y);
       xv[k][1] = make_float2(r.z, r.w);
     }
+    bool bad = false;
 #pragma unroll 2
     for (int o = 0; o < D; ++o) {
       const float4* wp = reinterpret_cast<const float4*>(ws + o * kFPairs);
@@ -268,9 +328,11 @@ __device__ __forceinline__ void pairs32(const FArgs& a, const FJob& job, int D, 
           fma2(acc[1], make_float2(wv[u], wv[u]), xv[k + u][1]);
         }
       }
+      if (o == 0) bad = not_finite(acc);
       reinterpret_cast<float4*>(z + (dst[o] + off) * 32)[h] =
           make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
     }
+    if (bad) redo_half(D, src, dst, ws, x + h * 16, z + h * 16, off);
   }
 }
 
@@ -428,7 +490,7 @@ std::shared_ptr<FactoredOp> build_tables(const System& sys, const Operator& op, 
         double v = V(x, y, x2, y2);
         if (y == y2) v += e1(x, x2) / kp;
         if (x == x2) v += e1(y, y2) / kn;
-        w.push_back(v);
+        w.push_back(std::fabs(v) >= kFDrop ? v : 0.0);
       }
   }
   // The species with fewer cores gives the jobs' cores and the other one the
@@ -514,7 +576,10 @@ std::shared_ptr<FactoredOp> build_tables(const System& sys, const Operator& op, 
       if (l.size() > 256) return nullptr;
       kv.second.w0 = uint32_t(w.size());
       for (uint16_t p : l)
-        for (uint16_t q : l) w.push_back(V(g0 + (p & 0xff), g0 + (p >> 8), g0 + (q & 0xff), g0 + (q >> 8)));
+        for (uint16_t q : l) {
+          const double v = V(g0 + (p & 0xff), g0 + (p >> 8), g0 + (q & 0xff), g0 + (q >> 8));
+          w.push_back(std::fabs(v) >= kFDrop ? v : 0.0);
+        }
     }
     const Cores two = make_cores(no, k - 2, m2 + g0, par + g0);
     for (auto& gr : two.group)
