@@ -565,8 +565,10 @@ void spmm_host(const Hamiltonian& h, int precision, const double* x, double* y, 
 // this matrix and, for up to 8 vectors, the factored and the block-tiled
 // product where they exist (CUDA events on the handle's stream, median of
 // `reps`); keep the fastest in h.tuning / h.format.  Returns the per-candidate
-// times (the tiled candidate carries ctas_per_sm = 0, the factored one -1).  Shapes with fewer than 16 resident warps per SM are not
-// tried (the gathers of the row-wise product need more in flight; they were
+// times (the tiled candidate carries ctas_per_sm = 0, the factored one -1).  More
+// than 8 vectors time the row-wise shapes alone and leave h.format, which products
+// of up to 8 and the solver's passes go by, as it is.  Shapes with fewer than 16
+// resident warps per SM are not tried (the gathers of the row-wise product need more in flight; they were
 // 2-6x slower than the best on every matrix measured), and a candidate whose
 // warm-up launch takes more than twice the best median so far is not
 // repeated.
@@ -605,6 +607,7 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
   std::vector<SpmmCandidate> out;
   const SpmmTuning keep = h.tuning;
   SpmmTuning bt = keep;
+  const int given = h.format;
   int best_format = CG_FORMAT_ROWS;
   h.format = CG_FORMAT_ROWS;
   for (int w : {4, 8, 16, 32})
@@ -647,7 +650,7 @@ std::vector<SpmmCandidate> spmm_autotune(Hamiltonian& h, int m, int reps) {
   }
   h.tuning = bt;
   h.tuning.tuned = true;
-  h.format = best_format;
+  h.format = m <= 8 ? best_format : given;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   return out;

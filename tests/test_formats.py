@@ -37,3 +37,20 @@ def test_on_the_fly_formats(gpu_available, space, nv, zv, twom, tmp_path):
     h.set_format(cg.CG_FORMAT_FACTORED)
     assert h.format_in_use() == cg.CG_FORMAT_FACTORED
     assert np.array_equal(h.times_matrix(x, cg.CG_PREC_FP32), y)
+
+
+@pytest.fixture(scope="module")
+def stored(tmp_path_factory):
+    """fp 2+4, 2M = 0: 3.3e7 stored entries, factored by default."""
+    p, b = _problem(tmp_path_factory.mktemp("fp24"), "fp", 2, 4, 0)
+    h = cg.Hamiltonian(p, b, cg.CG_PREC_FP32)
+    assert 2 ** 24 <= h.info.nnz_full < 2 ** 26 and h.format_in_use() == cg.CG_FORMAT_FACTORED
+    return p, b, h
+
+
+def test_autotune_of_wide_blocks_keeps_the_format(gpu_available, stored):
+    h = stored[2]
+    for fmt in (cg.CG_FORMAT_TILED, cg.CG_FORMAT_ROWS, cg.CG_FORMAT_FACTORED):
+        h.set_format(fmt)
+        r = h.autotune(16, reps=1)
+        assert r["format"] == h.format_in_use() == fmt and all(c[1] > 0 for c in r["candidates"])
