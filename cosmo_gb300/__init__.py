@@ -552,24 +552,9 @@ class Hamiltonian:
         if cache and os.path.exists(cache):
             with open(cache) as f:
                 db = json.load(f)
-            if key in db:
-                w, c = db[key]["warps"], db[key]["ctas_per_sm"]
-                _check(lib().cg_spmm_set_tuning(self._h, w, c))
-                fmt = db[key].get("format", CG_FORMAT_ROWS)
-                if fmt == CG_FORMAT_FACTORED:
-                    try:
-                        self.set_format(fmt)
-                    except CosmoError:  # no factored form of this matrix here
-                        fmt = CG_FORMAT_ROWS
-                elif fmt == CG_FORMAT_ROWS and self.format_in_use() == CG_FORMAT_FACTORED:
-                    self.set_format(fmt)
-                elif fmt == CG_FORMAT_TILED and not self.format()[1]:
-                    fmt = CG_FORMAT_ROWS
-                elif self.format()[1]:
-                    self.set_format(fmt)
-                    if "tiled_shape" in db[key]:
-                        self.set_tiled_shape(*db[key]["tiled_shape"])
-                return {"warps": w, "ctas_per_sm": c, "format": fmt, "cached": True}
+            if key in db and self._apply_tuning(db[key], nvec):
+                return {"warps": db[key]["warps"], "ctas_per_sm": db[key]["ctas_per_sm"],
+                        "format": self.format_in_use(), "cached": True}
         cap = C.c_int32(64)
         w = np.zeros(64, dtype=np.int32)
         c = np.zeros(64, dtype=np.int32)
@@ -585,13 +570,35 @@ class Hamiltonian:
             if os.path.exists(cache):
                 with open(cache) as f:
                     db = json.load(f)
-            db[key] = {"warps": bw, "ctas_per_sm": bc, "format": fmt, "ms": float(min(ms[:k]))}
+            timed = {0: CG_FORMAT_TILED, -1: CG_FORMAT_FACTORED}
+            db[key] = {"warps": bw, "ctas_per_sm": bc, "format": fmt, "ms": float(min(ms[:k])),
+                       "timed": sorted({timed.get(int(x), CG_FORMAT_ROWS) for x in c[:k]})}
             fi = self.format_info() if fmt != CG_FORMAT_FACTORED else {"tiled_available": False}
             if fi["tiled_available"]:
                 db[key]["tiled_shape"] = [fi["slices_per_warp"], fi["stages"]]
             with open(cache, "w") as f:
                 json.dump(db, f, indent=1, sort_keys=True)
         return res
+
+    def _apply_tuning(self, entry: dict, nvec: int) -> bool:
+        """Set a cached choice; False where it does not settle this matrix: the factored form is cached and does not
+        exist here, or it does and was not among the formats timed."""
+        if nvec <= 8:
+            fmt, given = entry.get("format", CG_FORMAT_ROWS), self.format_in_use()
+            if given == CG_FORMAT_FACTORED and given not in entry.get("timed", [fmt]):
+                return False
+            if fmt == CG_FORMAT_FACTORED:
+                try:
+                    self.set_format(fmt)
+                except CosmoError:
+                    return False
+            else:
+                tiled = (fmt == CG_FORMAT_TILED or given != CG_FORMAT_FACTORED) and self.format()[1]
+                self.set_format(fmt if tiled else CG_FORMAT_ROWS)
+                if tiled and "tiled_shape" in entry:
+                    self.set_tiled_shape(*entry["tiled_shape"])
+        _check(lib().cg_spmm_set_tuning(self._h, entry["warps"], entry["ctas_per_sm"]))
+        return True
 
     def tuning(self):
         w, c, t = C.c_int32(), C.c_int32(), C.c_int32()

@@ -2,11 +2,14 @@
 switched off and on again, on on-the-fly and on stored matrices.  Every format
 within 1e-5 of max |y| of the FP64 product; the formats' own results come back
 bit by bit when they are chosen again."""
+import json
+
 import numpy as np
 import pytest
 
 import cosmo_gb300 as cg
 from cosmo_gb300.synthetic import SyntheticSystem, make_system
+from conftest import problem_for
 from test_factored import SYSTEMS
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +57,44 @@ def test_autotune_of_wide_blocks_keeps_the_format(gpu_available, stored):
         h.set_format(fmt)
         r = h.autotune(16, reps=1)
         assert r["format"] == h.format_in_use() == fmt and all(c[1] > 0 for c in r["candidates"])
+
+
+def test_tuning_cache_and_the_factored_form(gpu_available, stored, tmp_path):
+    """A cached choice is reused where it settles the matrix and timed again where it does not."""
+    h, cache = stored[2], str(tmp_path / "tune.json")
+
+    def edit(**kw):
+        with open(cache) as f:
+            db = json.load(f)
+        (key, entry), = db.items()
+        entry.update(kw)
+        for k in [k for k, v in kw.items() if v is None]:
+            del entry[k]
+        with open(cache, "w") as f:
+            json.dump({key: entry}, f)
+
+    h.set_format(cg.CG_FORMAT_FACTORED)
+    first = h.autotune(8, reps=1, cache=cache)
+    assert first["cached"] is False and any(c[1] == -1 for c in first["candidates"])
+    h.set_format(cg.CG_FORMAT_FACTORED)
+    again = h.autotune(8, reps=1, cache=cache)
+    assert again["cached"] is True and again["format"] == first["format"] == h.format_in_use()
+    # an entry from before the factored form existed
+    for fmt in (cg.CG_FORMAT_ROWS, cg.CG_FORMAT_TILED):
+        h.set_format(cg.CG_FORMAT_FACTORED)
+        edit(format=fmt, timed=None)
+        assert h.autotune(8, reps=1, cache=cache)["cached"] is False
+        assert h.autotune(8, reps=1, cache=cache)["cached"] is True
+    # an entry whose factored form does not exist for this handle
+    small = cg.Hamiltonian(*(lambda p: (p, cg.ManyBodyStates(p)))(problem_for("sd44m0s4", str(tmp_path))), cg.CG_PREC_FP32)
+    cache = str(tmp_path / "small.json")
+    assert small.autotune(8, reps=1, cache=cache)["cached"] is False
+    edit(format=cg.CG_FORMAT_FACTORED)
+    r = small.autotune(8, reps=1, cache=cache)
+    assert r["cached"] is False and r["format"] == small.format_in_use() == cg.CG_FORMAT_ROWS
+    # choices for wide blocks leave the format of narrow ones alone
+    h.set_format(cg.CG_FORMAT_FACTORED)
+    cache = str(tmp_path / "wide.json")
+    for cached in (False, True):
+        r = h.autotune(16, reps=1, cache=cache)
+        assert r["cached"] is cached and r["format"] == h.format_in_use() == cg.CG_FORMAT_FACTORED
