@@ -795,7 +795,11 @@ cg_status cg_spmm_get_format(const cg_hamiltonian* h, cg_spmm_format_info* info)
     CG_NOT_NULL(h);
     CG_NOT_NULL(info);
     *info = cg_spmm_format_info{};
-    tiled_on_demand(h);
+    try {
+      tiled_on_demand(h);
+    } catch (const cg::Error& e) {  // a question: no room for the copy means there is none
+      if (e.code != CG_ERR_NOMEM) throw;
+    }
     const cg::TiledOp* t = h->h.tiled.get();
     info->format = format_in_use(h->h);
     info->tiled_available = t != nullptr;

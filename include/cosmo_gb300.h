@@ -258,7 +258,8 @@ cg_status cg_spmm_get_tuning(const cg_hamiltonian* h, int32_t* warps, int32_t* c
  * (PPMatrix2CSBBlk, include/sm/PPMatrix.cxx:571-656); the choice of format has
  * no counterpart there.  From 2^26 stored entries up the copy is built with the
  * matrix, or when first asked about (cg_spmm_get_format, cg_spmm_set_format,
- * cg_spmm_set_tiled_shape) if the matrix uses its factored form; below, on
+ * cg_spmm_set_tiled_shape) if the matrix uses its factored form (the query
+ * answers tiled_available = 0 where it does not fit); below, on
  * request (cg_spmm_set_format(h, CG_FORMAT_TILED)).  cg_spmm_autotune picks the
  * fastest of the formats that exist (its tiled candidate is reported with
  * ctas_per_sm = 0, the factored one with -1). */

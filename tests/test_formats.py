@@ -11,6 +11,7 @@ import cosmo_gb300 as cg
 from cosmo_gb300.synthetic import SyntheticSystem, make_system
 from conftest import problem_for
 from test_factored import SYSTEMS
+from test_work_area import _full
 
 pytestmark = pytest.mark.gpu
 
@@ -98,3 +99,13 @@ def test_tuning_cache_and_the_factored_form(gpu_available, stored, tmp_path):
     for cached in (False, True):
         r = h.autotune(16, reps=1, cache=cache)
         assert r["cached"] is cached and r["format"] == h.format_in_use() == cg.CG_FORMAT_FACTORED
+
+
+def test_query_on_a_full_device(gpu_available, tmp_path):
+    """The block-tiled copy that a query would make (2.5e8 entries) does not fit: the answer is that there is none."""
+    p, b = _problem(tmp_path, "fp", 3, 4, 1)
+    h = cg.Hamiltonian(p, b, cg.CG_PREC_FP32)
+    assert h.format_in_use() == cg.CG_FORMAT_FACTORED
+    with _full(256 << 20):
+        assert h.format()[:2] == (cg.CG_FORMAT_FACTORED, False)
+    assert h.format()[:2] == (cg.CG_FORMAT_FACTORED, True)
