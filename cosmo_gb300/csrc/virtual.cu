@@ -696,7 +696,7 @@ bool Hamiltonian::release_work() const {
 
 uint64_t Hamiltonian::device_bytes() const {
   return rowptr.bytes() + col.bytes() + val64.bytes() + hi.bytes() + lo.bytes() + diag.bytes() +
-         (virt ? virt->bytes() : 0) + (fact ? fact->bytes() : 0) + (tiled ? tiled->bytes() : 0);
+         host_work.bytes() + (virt ? virt->bytes() : 0) + (fact ? fact->bytes() : 0) + (tiled ? tiled->bytes() : 0);
 }
 
 // ------------------------------------------------------------------- build

@@ -105,3 +105,14 @@ def test_full_device(gpu_available, problem):
     with _full(AREA + (220 << 20)):
         np.testing.assert_allclose(_solve(h), eig, rtol=0, atol=1e-6)
         assert h.format_in_use() == cg.CG_FORMAT_ROWS
+
+
+def test_host_buffers_are_counted(gpu_available, tmp_path):
+    """Host products keep their device buffers with the handle (FP64, 4 vectors: the block and two operands)."""
+    p = cg.Problem(make_system(str(tmp_path), SyntheticSystem("sd", 4, 4, 0, "+", 0.5, 31))[1])
+    b = cg.ManyBodyStates(p)
+    for virtual in (False, True):
+        h = cg.Hamiltonian(p, b, cg.CG_PREC_FP64, virtual=virtual)
+        bare = _bytes(h)
+        h.times_matrix(np.ones((b.n, 4)))
+        assert _bytes(h) - bare >= 3 * b.n * 4 * 8
