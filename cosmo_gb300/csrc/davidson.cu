@@ -1771,13 +1771,7 @@ DavResult davidson_solve(const Hamiltonian& h, const DavidsonRequest& rq) {
     const FactoredOp* f;
     ~Area() { if (f) f->z.release(); }
   } area{h.virt && h.fact && !h.fact->z.p ? h.fact.get() : nullptr};
-  try {
-    return solve(h, rq);
-  } catch (const Error& e) {
-    if (e.code != CG_ERR_NOMEM || !h.release_work()) throw;
-    h.fact_failed = h.fact != nullptr;
-    return solve(h, rq);
-  }
+  return with_room(h, [&] { return solve(h, rq); });
 }
 
 }  // namespace cg

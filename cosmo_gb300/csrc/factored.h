@@ -82,6 +82,19 @@ constexpr uint64_t kFactoredMinEntries = 1ull << 24;
 // built, an on-the-fly one with its first FP32 product: the path is there for
 // problems that fill the device, and a solve's vectors come first.
 bool factored_ready(const Hamiltonian& h);
+// f(), and where its memory runs out, once more without what products keep
+// (that product then stays with the one the factored form replaced).
+template <class F>
+auto with_room(const Hamiltonian& h, F&& f) {
+  try {
+    return f();
+  } catch (const Error& e) {
+    const bool area = h.fact && h.fact->z.p;
+    if (e.code != CG_ERR_NOMEM || !h.release_work()) throw;
+    h.fact_failed |= area;
+    return f();
+  }
+}
 
 // Y = H X from x packed as n rows of 8 FP32 vectors (32-byte aligned).
 // Asynchronous; allocates nothing (factored_ready has been called).

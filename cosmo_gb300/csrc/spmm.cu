@@ -557,8 +557,10 @@ void spmm_host_t(const Hamiltonian& h, int precision, const double* x, double* y
 
 void spmm_host(const Hamiltonian& h, int precision, const double* x, double* y, int m) {
   if (m < 1) throw Error(CG_ERR_ARG, "m must be >= 1");
-  if (precision == CG_PREC_FP32) spmm_host_t<float>(h, precision, x, y, m);
-  else spmm_host_t<double>(h, precision, x, y, m);
+  with_room(h, [&] {
+    if (precision == CG_PREC_FP32) spmm_host_t<float>(h, precision, x, y, m);
+    else spmm_host_t<double>(h, precision, x, y, m);
+  });
 }
 
 // Autotuner: time every candidate launch shape of the row-wise FP32 product on

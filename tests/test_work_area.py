@@ -116,3 +116,17 @@ def test_host_buffers_are_counted(gpu_available, tmp_path):
         bare = _bytes(h)
         h.times_matrix(np.ones((b.n, 4)))
         assert _bytes(h) - bare >= 3 * b.n * 4 * 8
+
+
+def test_host_product_beside_the_area(gpu_available, problem):
+    """An FP64 host product whose buffers fit only in place of the area that FP32 products left."""
+    b = problem[1]
+    h = cg.Hamiltonian(*problem, cg.CG_PREC_FP32, virtual=True)
+    x = np.random.default_rng(4).standard_normal((b.n, 8))
+    y32 = h.times_matrix(x, cg.CG_PREC_FP32)
+    with _full(16 << 20):  # and the FP32 call's buffers, 62 MB; FP64 takes 93
+        y = h.times_matrix(x, cg.CG_PREC_FP64)
+        assert h.format_in_use() == cg.CG_FORMAT_ROWS
+    assert np.abs(y32 - y).max() <= 1e-5 * np.abs(y).max()
+    h.set_format(cg.CG_FORMAT_FACTORED)
+    assert np.array_equal(h.times_matrix(x, cg.CG_PREC_FP32), y32)
