@@ -21,11 +21,12 @@ inline void axpy_rows(int m, int rows, const double* f, const double* a, size_t 
     for (int j = 0; j < m; ++j) y[j] += f0 * a0[j];
   }
 }
-inline void rotate(int m, double c, double s, double* __restrict__ x, double* __restrict__ y) {
+// rows (x, y) <- (c x + s y, c y - s x)
+inline void turn(int m, double c, double s, double* __restrict__ x, double* __restrict__ y) {
   for (int k = 0; k < m; ++k) {
-    const double f = y[k];
-    y[k] = s * x[k] + c * f;
-    x[k] = c * x[k] - s * f;
+    const double u = x[k], v = y[k];
+    x[k] = c * u + s * v;
+    y[k] = c * v - s * u;
   }
 }
 }  // namespace
@@ -99,46 +100,44 @@ inline void reflect(int n, const std::vector<double>& z, const std::vector<doubl
   }
 }
 
-// Implicit QL with Wilkinson shifts on (d, e); the rotations act on the rows
-// of q (n x n, nullptr: eigenvalues only).  d is not sorted.
-void ql(int n, std::vector<double>& d, std::vector<double>& e, double* q) {
+// Diagonalises the tridiagonal (d, e) in place by QR steps with an implicit
+// shift (Golub & Van Loan, Matrix Computations, section 8.3): the shift is the
+// eigenvalue of the trailing 2 x 2 block nearer to its last element, the first
+// plane rotation is the one that T - shift asks for, and every further one
+// chases the element it leaves outside the band one row down.  The rotations
+// act on the rows of q (n x n, nullptr: eigenvalues only).  d is not sorted.
+void shifted_qr(int n, std::vector<double>& d, std::vector<double>& e, double* q) {
   const size_t ld = size_t(n);
-  for (int l = 0; l < n; ++l) {
-    int iter = 0, m;
-    do {
-      for (m = l; m < n - 1; ++m) {
-        double dd = std::fabs(d[m]) + std::fabs(d[m + 1]);
-        if (std::fabs(e[m]) <= 1e-16 * dd) break;
+  constexpr int kMaxSteps = 60;  // for one eigenvalue; two or three are usual
+  const auto decoupled = [&](int i) { return std::fabs(e[i]) <= 1e-16 * (std::fabs(d[i]) + std::fabs(d[i + 1])); };
+  int steps = 0;
+  for (int last = n - 1; last > 0;) {
+    if (decoupled(last - 1) || ++steps > kMaxSteps) {
+      --last;
+      steps = 0;
+      continue;
+    }
+    int first = last - 1;
+    while (first > 0 && !decoupled(first - 1)) --first;
+    const double half = 0.5 * (d[last - 1] - d[last]), off = e[last - 1];
+    const double shift = d[last] - off * (off / (half + std::copysign(std::hypot(half, off), half)));
+    double in = d[first] - shift, out = e[first];  // the pair whose second part the rotation removes
+    for (int k = first; k < last; ++k) {
+      const double len = std::hypot(in, out);
+      const double c = len > 0.0 ? in / len : 1.0, s = len > 0.0 ? out / len : 0.0;
+      if (k > first) e[k - 1] = len;
+      const double gap = d[k + 1] - d[k], b = e[k];
+      const double move = s * (s * gap + 2.0 * c * b);
+      d[k] += move;
+      d[k + 1] -= move;
+      e[k] = c * s * gap + (c - s) * (c + s) * b;
+      if (q) turn(n, c, s, q + k * ld, q + (k + 1) * ld);
+      if (k + 1 < last) {
+        in = e[k];
+        out = s * e[k + 1];
+        e[k + 1] *= c;
       }
-      if (m != l) {
-        if (++iter > 60) break;
-        double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-        double r = std::hypot(g, 1.0);
-        g = d[m] - d[l] + e[l] / (g + (g >= 0.0 ? std::fabs(r) : -std::fabs(r)));
-        double s = 1.0, c = 1.0, pp = 0.0;
-        int i;
-        for (i = m - 1; i >= l; --i) {
-          double f = s * e[i], b = c * e[i];
-          e[i + 1] = (r = std::hypot(f, g));
-          if (r == 0.0) {
-            d[i + 1] -= pp;
-            e[m] = 0.0;
-            break;
-          }
-          s = f / r;
-          c = g / r;
-          g = d[i + 1] - pp;
-          r = (d[i] - g) * s + 2.0 * c * b;
-          d[i + 1] = g + (pp = s * r);
-          g = c * r - b;
-          if (q) rotate(n, c, s, q + i * ld, q + (i + 1) * ld);
-        }
-        if (r == 0.0 && i >= l) continue;
-        d[l] -= pp;
-        e[l] = g;
-        e[m] = 0.0;
-      }
-    } while (m != l);
+    }
   }
 }
 
@@ -234,11 +233,10 @@ bool inverse_iteration(int n, const std::vector<double>& d, const std::vector<do
 }
 }  // namespace
 
-// Householder reduction and implicit QL from the textbook algorithms
-// (Wilkinson & Reinsch, Handbook for Automatic Computation II), the inner
-// loops along rows.  need < n: only that many lowest eigenvectors are formed,
-// by inverse iteration on the tridiagonal matrix (the QL then runs without
-// vectors); the other columns of zout are zero.  One such problem per Davidson
+// Householder reduction (Wilkinson & Reinsch, Handbook for Automatic Computation
+// II) and shifted QR steps, the inner loops along rows.  need < n: only that
+// many lowest eigenvectors are formed, by inverse iteration on the tridiagonal
+// matrix (the QR steps then run without vectors); the other columns of zout are zero.  One such problem per Davidson
 // iteration (up to 96 x 96): 24 -> 11 ms of a 46 -> 33 ms solve of 62 iterations
 // (sd 4+4).
 void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::vector<double>& zout, int need) {
@@ -251,7 +249,7 @@ void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::v
   zout.assign(ld * n, 0.0);
   if (need >= 0 && 2 * need < n && n >= 16) {
     std::vector<double> dq(d), eq(e), v;
-    ql(n, dq, eq, nullptr);
+    shifted_qr(n, dq, eq, nullptr);
     std::sort(dq.begin(), dq.end());
     if (inverse_iteration(n, d, e, dq, need, v)) {
       w = dq;
@@ -266,7 +264,7 @@ void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::v
   std::vector<double> q(ld * n, 0.0);
   for (int i = 0; i < n; ++i) q[i * ld + i] = 1.0;
   for (int i = 0; i < n; ++i) reflect(n, z, hs, &q[i * ld]);
-  ql(n, d, e, q.data());
+  shifted_qr(n, d, e, q.data());
   std::vector<int> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
   std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return d[x] < d[y]; });

@@ -8,8 +8,8 @@ namespace cg {
 // Eigen-decomposition of the symmetric n x n matrix a (row-major, n*n).
 // On return w holds the eigenvalues in ascending order and z (row-major, n*n)
 // the eigenvectors as columns: z[i*n + k] is component i of eigenvector k.
-// Householder tridiagonalisation followed by the implicit QL iteration, the
-// method of tav::EigenSystemT (include/tav/EigenSystem.cxx:49-69).
+// Householder tridiagonalisation followed by an implicitly shifted iteration, as
+// in tav::EigenSystemT (include/tav/EigenSystem.cxx:49-69).
 // need >= 0: only the need lowest eigenvectors are wanted; columns of z beyond
 // them may be zero.
 void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::vector<double>& z, int need = -1);
