@@ -100,42 +100,44 @@ inline void reflect(int n, const std::vector<double>& z, const std::vector<doubl
   }
 }
 
-// Diagonalises the tridiagonal (d, e) in place by QR steps with an implicit
-// shift (Golub & Van Loan, Matrix Computations, section 8.3): the shift is the
-// eigenvalue of the trailing 2 x 2 block nearer to its last element, the first
-// plane rotation is the one that T - shift asks for, and every further one
-// chases the element it leaves outside the band one row down.  The rotations
-// act on the rows of q (n x n, nullptr: eigenvalues only).  d is not sorted.
-void shifted_qr(int n, std::vector<double>& d, std::vector<double>& e, double* q) {
+// Diagonalises the tridiagonal (d, e) in place by implicitly shifted steps
+// (Golub & Van Loan, Matrix Computations, section 8.3, upside down: the small
+// eigenvalues of a projected problem come to the top and decouple first): the
+// shift is the eigenvalue of the leading 2 x 2 block nearer to its first
+// element, the first plane rotation is the one that T - shift asks for in the
+// last two rows, and every further one chases the element left outside the band
+// one row up.  The rotations act on the rows of q (n x n, nullptr: eigenvalues
+// only).  d is not sorted.
+void shifted_steps(int n, std::vector<double>& d, std::vector<double>& e, double* q) {
   const size_t ld = size_t(n);
   constexpr int kMaxSteps = 60;  // for one eigenvalue; two or three are usual
   const auto decoupled = [&](int i) { return std::fabs(e[i]) <= 1e-16 * (std::fabs(d[i]) + std::fabs(d[i + 1])); };
   int steps = 0;
-  for (int last = n - 1; last > 0;) {
-    if (decoupled(last - 1) || ++steps > kMaxSteps) {
-      --last;
+  for (int first = 0; first + 1 < n;) {
+    if (decoupled(first) || ++steps > kMaxSteps) {
+      ++first;
       steps = 0;
       continue;
     }
-    int first = last - 1;
-    while (first > 0 && !decoupled(first - 1)) --first;
-    const double half = 0.5 * (d[last - 1] - d[last]), off = e[last - 1];
-    const double shift = d[last] - off * (off / (half + std::copysign(std::hypot(half, off), half)));
-    double in = d[first] - shift, out = e[first];  // the pair whose second part the rotation removes
-    for (int k = first; k < last; ++k) {
+    int last = first + 1;
+    while (last + 1 < n && !decoupled(last)) ++last;
+    const double half = 0.5 * (d[first + 1] - d[first]), off = e[first];
+    const double shift = d[first] - off * (off / (half + std::copysign(std::hypot(half, off), half)));
+    double in = d[last] - shift, out = e[last - 1];  // the pair whose second part the rotation removes
+    for (int k = last; k > first; --k) {             // rows k and k - 1
       const double len = std::hypot(in, out);
       const double c = len > 0.0 ? in / len : 1.0, s = len > 0.0 ? out / len : 0.0;
-      if (k > first) e[k - 1] = len;
-      const double gap = d[k + 1] - d[k], b = e[k];
-      const double move = s * (s * gap + 2.0 * c * b);
-      d[k] += move;
-      d[k + 1] -= move;
-      e[k] = c * s * gap + (c - s) * (c + s) * b;
-      if (q) turn(n, c, s, q + k * ld, q + (k + 1) * ld);
-      if (k + 1 < last) {
-        in = e[k];
-        out = s * e[k + 1];
-        e[k + 1] *= c;
+      if (k < last) e[k] = len;
+      // the 2 x 2 block [u b; b v] turned: u + s t, v - s t and c t - b with t = s (v - u) + 2 c b
+      const double b = e[k - 1], t = s * (d[k - 1] - d[k]) + 2.0 * c * b;
+      d[k] += s * t;
+      d[k - 1] -= s * t;
+      e[k - 1] = c * t - b;
+      if (q) turn(n, c, s, q + k * ld, q + (k - 1) * ld);
+      if (k - 1 > first) {
+        in = e[k - 1];
+        out = s * e[k - 2];
+        e[k - 2] *= c;
       }
     }
   }
@@ -234,9 +236,9 @@ bool inverse_iteration(int n, const std::vector<double>& d, const std::vector<do
 }  // namespace
 
 // Householder reduction (Wilkinson & Reinsch, Handbook for Automatic Computation
-// II) and shifted QR steps, the inner loops along rows.  need < n: only that
-// many lowest eigenvectors are formed, by inverse iteration on the tridiagonal
-// matrix (the QR steps then run without vectors); the other columns of zout are zero.  One such problem per Davidson
+// II) and shifted steps, the inner loops along rows.  need < n: only that many
+// lowest eigenvectors are formed, by inverse iteration on the tridiagonal matrix
+// (the steps then run without vectors); the other columns of zout are zero.  One such problem per Davidson
 // iteration (up to 96 x 96): 24 -> 11 ms of a 46 -> 33 ms solve of 62 iterations
 // (sd 4+4).
 void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::vector<double>& zout, int need) {
@@ -249,7 +251,7 @@ void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::v
   zout.assign(ld * n, 0.0);
   if (need >= 0 && 2 * need < n && n >= 16) {
     std::vector<double> dq(d), eq(e), v;
-    shifted_qr(n, dq, eq, nullptr);
+    shifted_steps(n, dq, eq, nullptr);
     std::sort(dq.begin(), dq.end());
     if (inverse_iteration(n, d, e, dq, need, v)) {
       w = dq;
@@ -264,7 +266,7 @@ void sym_eig(int n, const std::vector<double>& a, std::vector<double>& w, std::v
   std::vector<double> q(ld * n, 0.0);
   for (int i = 0; i < n; ++i) q[i * ld + i] = 1.0;
   for (int i = 0; i < n; ++i) reflect(n, z, hs, &q[i * ld]);
-  shifted_qr(n, d, e, q.data());
+  shifted_steps(n, d, e, q.data());
   std::vector<int> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
   std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return d[x] < d[y]; });

@@ -494,7 +494,7 @@ cg_status cg_xlevels(const char* const* files, int32_t nfiles, const char* out_x
  * n, state k at vecs + k*n, or NULL).  The path the reference's DXHV takes
  * instead of Davidson when the dimension is at most its limit
  * (include/xsm/DEXHVcsb.cxx:80-110, Eigen's SelfAdjointEigenSolver; here the
- * Householder + shifted QR solver of the Davidson's projected problems on
+ * Householder + shifted-step solver of the Davidson's projected problems on
  * the host).  Stored matrices only (CG_ERR_UNSUPPORTED on the fly), n <= 8192
  * (CG_ERR_ARG above); eigenvector signs are the solver's own. */
 cg_status cg_dense_eigensolve(const cg_hamiltonian* h, double* eig, double* vecs);
