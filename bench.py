@@ -654,7 +654,8 @@ def virtual_subbench(cg, fp64_iters):
             "n": int(n), "connections_per_product": conn, "table_bytes": int(hv.info.device_bytes),
             "setup_seconds": setup, "fp32_product_ms_8vec": ms32, "fp64_product_ms_4vec": ms64,
             "double_float_product_ms_4vec": msdf,
-            "product_timing_note": "device API calls: pack kernel + product, staging buffer allocated per call",
+            "product_timing_note": "device API calls on operands that need no packing (FP32 8, FP64 4 vectors); "
+                                   "double-float with its pack kernel",
             "fp32_connection_vectors_per_s": conn * 8 / (ms32 * 1e-3),
             "fp64_connection_vectors_per_s": conn * 4 / (ms64 * 1e-3),
             "mixed_solve_seconds": mixed, "mixed_iterations": int(r.stats.iterations),

@@ -68,7 +68,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // FP32 product of 8 vectors, neutron + proton pairs.  Bound by the FP32 pipe in
 // principle (fp 4 + 4: 1.7e9 multiply-adds x 8 with filled-up tiles, 0.35 ms); it
-// takes 0.84 ms, the rest waiting at the two barriers of a chunk.  Four warps a
+// takes 0.85 ms, the rest waiting at the two barriers of a chunk.  Four warps a
 // CTA and four CTAs an SM measured best (3, 5, 6, 8 warps with tiles of 8: 1.00,
 // 0.91, 0.98, 1.10 ms against 0.89; rows fetched in two alternating halves 0.90).
 // A warp forms tiles of 2 groups of OT <= 8 outputs x 16 spectators (fact_tiles).
@@ -90,7 +90,7 @@ struct alignas(16) FHead32 {
 // matrix, where the element-wise products reach connected rows only.  It shows
 // in any one output: where that is not finite, all are formed again without the
 // zeros (an infinity still comes out as NaN where the terms of an element differ
-// in sign).
+// in sign).  fp 4 + 4: 1.367 -> 1.377 ms a product.
 template <int N>
 __device__ __forceinline__ bool not_finite(const float2 (&v)[N]) {
   float2 c = make_float2(0.f, 0.f);
@@ -185,7 +185,7 @@ __device__ __forceinline__ void tile32(const FArgs& a, const FHead32& hd, int D,
 
 // Outputs of a job in 1, 2 or 4 warp tiles (more above 64 pairs) of 2 groups of
 // OT, as even as they can be: with tiles of 16 one of the four warps was idle
-// for 33 to 48 pairs, half of the work of fp 4 + 4 (0.89 ms; now 0.84).
+// for 33 to 48 pairs, half of the work of fp 4 + 4 (0.89 ms; so 0.84).
 __host__ __device__ inline int fact_tiles(int D) { return D <= 16 ? 1 : D <= 32 ? 2 : D <= 64 ? 4 : (D + 15) / 16; }
 
 __global__ void __launch_bounds__(kFW * 32, 4) k_fact32(FArgs a, const float* __restrict__ w,

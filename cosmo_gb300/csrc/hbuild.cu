@@ -625,7 +625,8 @@ void hamiltonian_build(const System& sys, const Operator& op, const Basis& b, in
     // faster than the stored values: 3.4 us per million entries row-wise, 1.9 us
     // block-tiled with long blocks and more with short ones (fp 4+4, 405 rows a
     // block: 2.42 ms tiled, 1.37 factored; fp 4+3, 100 rows: 0.59 and 0.27; fp 5+2,
-    // 17 rows: 0.54, row-wise 0.41 and 0.23; fp 3+3: row-wise 0.16 and 0.07)
+    // 17 rows: 0.54, row-wise 0.41 and 0.23; fp 3+3: row-wise 0.16 and 0.07).  The
+    // tiled figure is for kTiledMinEntries and more (fewer take longer: tiled.h)
     const auto t0 = std::chrono::steady_clock::now();
     const double per_block = double(n) / double(std::max<size_t>(b.h_bstart.size(), 1));
     const double per_entry = h.nnz >= kTiledMinEntries ? std::min(3.4e-6, 1.9e-6 * (1 + 40 / per_block)) : 3.4e-6;

@@ -50,8 +50,9 @@ struct TiledOp {
 };
 
 // Stored entries from which an FP32 matrix built from a basis gets its tiled
-// copy by default (below, the row-wise kernel is as fast and the copy is
-// built on request, cg_spmm_set_format).
+// copy by default.  Below, the row-wise kernel is as fast or faster (8 vectors,
+// row-wise / block-tiled at its best shape: sd 6+6, 2.5e7 entries, 104 / 112 us,
+// fp 2+4, 3.3e7, 138 / 137) and the copy is built on request (cg_spmm_set_format).
 constexpr uint64_t kTiledMinEntries = uint64_t(1) << 26;
 // Longest block the product's shared-memory staging takes.
 constexpr int kTiledMaxBlock = 1536;
